@@ -29,8 +29,9 @@ LIB = os.path.join(HERE, "libsodecl_cuda.so")
 GENCODE = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CUDA_SOURCES = ["aux_kernels.cu", "batch_noalloc.cu"]
 
-EMBED = [("kFastDivSrc", "fastdiv.cuh"), ("kPreludeSrc", "prelude.cuh"), ("kThreefrySrc", "threefry.cuh"),
-         ("kSolversSrc", "solvers.cuh"), ("kBatchSrc", "batch.cuh"), ("kAdjointSrc", "adjoint.cuh")]
+EMBED = [("kFastDivSrc", "fastdiv.cuh"), ("kPreludeSrc", "prelude.cuh"), ("kMathCoreSrc", "mathcore.cuh"),
+         ("kFastMathSrc", "fastmath.cuh"), ("kThreefrySrc", "threefry.cuh"), ("kSolversSrc", "solvers.cuh"),
+         ("kBatchSrc", "batch.cuh"), ("kAdjointSrc", "adjoint.cuh")]
 
 
 def _run(cmd, verbose):

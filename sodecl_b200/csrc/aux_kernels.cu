@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "device/fastdiv.cuh"
+#include "device/mathcore.cuh"
 #include "device/threefry.cuh"
 #include "sodecl_cuda.h"
 

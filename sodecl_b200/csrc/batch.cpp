@@ -121,7 +121,7 @@ int load_program(sodecl_batch *b, const std::vector<int> &lanes, int reg_blocks)
         b->lib = nullptr;
         b->kernel = nullptr;
         BATCH_TRY(b, cudaLibraryLoadData(&b->lib, b->prog->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-        BATCH_TRY(b, cudaLibraryGetKernel(&b->kernel, b->lib, b->prog->kernel_name.c_str()));
+        BATCH_TRY(b, sodecl_b200_batch::kernel_of(*b->prog, b->lib, &b->kernel));
     }
     while (b->block > 32 && sodecl_b200_batch::shared_bytes(b, b->block) > sodecl_b200_batch::kSharedCap)
         b->block -= 32;
@@ -273,7 +273,7 @@ int sodecl_batch_set_items(sodecl_batch *b, int64_t n, const int32_t *item_class
     }
     if (!b->lib) {
         BATCH_TRY(b, cudaLibraryLoadData(&b->lib, b->prog->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-        BATCH_TRY(b, cudaLibraryGetKernel(&b->kernel, b->lib, b->prog->kernel_name.c_str()));
+        BATCH_TRY(b, sodecl_b200_batch::kernel_of(*b->prog, b->lib, &b->kernel));
         BATCH_TRY(b, cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
         BATCH_TRY(b, cudaMalloc(&b->d_head, sizeof(unsigned long long) * kMaxClasses));
     }

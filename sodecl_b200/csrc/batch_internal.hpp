@@ -118,12 +118,23 @@ struct sodecl_batch {
 
 namespace sodecl_b200_batch {
 
-// Dynamic shared memory of one block of the batch kernel, and its cap (the
-// default limit, no opt-in).
+// Dynamic shared memory of one block of the batch kernel, and its cap.
 constexpr size_t kSharedCap = 48 * 1024;
 inline size_t shared_bytes(const sodecl_batch *b, int block)
 {
     return static_cast<size_t>(block / 32) * static_cast<size_t>(b->warp_words) * sizeof(double);
+}
+
+// The program's kernel from its loaded library.  Speculative programs keep
+// their threads' flags in static shared memory, so a launch at the cap goes
+// past the 48 KiB a block gets without asking.
+inline cudaError_t kernel_of(const sodecl_b200::Program &prog, cudaLibrary_t lib, cudaKernel_t *kernel)
+{
+    cudaError_t e = cudaLibraryGetKernel(kernel, lib, prog.kernel_name.c_str());
+    if (e == cudaSuccess && prog.speculate)
+        e = cudaFuncSetAttribute(reinterpret_cast<const void *>(*kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kSharedCap));
+    return e;
 }
 
 }  // namespace sodecl_b200_batch

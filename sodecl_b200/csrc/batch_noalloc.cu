@@ -109,7 +109,7 @@ extern "C" int sodecl_batch_run_noalloc(sodecl_batch *b, const sodecl_batch_io *
         if (!b->noalloc_kernel) {
             if (cudaLibraryLoadData(&b->noalloc_lib, b->prog->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) !=
                     cudaSuccess ||
-                cudaLibraryGetKernel(&b->noalloc_kernel, b->noalloc_lib, b->prog->kernel_name.c_str()) != cudaSuccess) {
+                sodecl_b200_batch::kernel_of(*b->prog, b->noalloc_lib, &b->noalloc_kernel) != cudaSuccess) {
                 const cudaError_t e = cudaGetLastError();
                 return fail(b, SODECL_ERR_CUDA, std::string("no-alloc run: loading the program: ") + cudaGetErrorString(e));
             }

@@ -172,8 +172,10 @@ __device__ __forceinline__ void sodecl_class_run(const sodecl_batch_args &a, con
     while (__any_sync(0xffffffffu, item >= 0)) {
         if (item >= 0) {
             if (left > 0) {
-                sodecl_advance(t, y, p, a.orbit_id ? a.orbit_id[item] : item, counter, passes, capped);
-                --left;
+                // one step, or in speculative classes a run of steps
+                const int m = SODECL_SPECULATE ? (int)min(left, (long long)SODECL_SPEC_RUN) : 1;
+                sodecl_advance_run(t, y, p, a.orbit_id ? a.orbit_id[item] : item, counter, passes, capped, m);
+                left -= m;
             }
             if (left <= 0) {
                 // store this orbit, take the next one (a count below zero
@@ -240,8 +242,15 @@ __device__ __forceinline__ void sodecl_class_run(const sodecl_batch_args &a, con
         const sodecl_i64 gid = a.orbit_id ? a.orbit_id[item] : item;
         sodecl_i64 passes = 0;
         int capped = 0;
+#if SODECL_SPECULATE
+#pragma unroll 1
+        for (long long s = 0; s < left; s += SODECL_SPEC_RUN)
+            sodecl_lanes_advance_run(t, yown, v, gid, counter, passes, capped,
+                                     (int)min(left - s, (long long)SODECL_SPEC_RUN));
+#else
 #pragma unroll 1
         for (long long s = 0; s < left; ++s) sodecl_lanes_advance(t, yown, v, gid, counter, passes, capped);
+#endif
         int nonfinite = 0;
 #pragma unroll
         for (int q = 0; q < SODECL_ROWS; ++q) {

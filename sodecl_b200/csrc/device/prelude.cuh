@@ -25,7 +25,10 @@ typedef double sodecl_num_t;
 // contraction and results are unchanged).  Conversions out of it are
 // explicit, so mixed expressions stay unambiguous; a system file that needs an
 // implicit conversion fails to compile with it and the front end builds the
-// plain program instead.
+// plain program instead.  The type has a namespace of its own, so that `/` is
+// looked up where the system file stands and not through its operands: the
+// speculative copy's namespace declares its own (fastmath.cuh).
+namespace sodecl_numeric {
 struct sodecl_num {
     sodecl_num_t v;
     __device__ __forceinline__ sodecl_num() = default;
@@ -48,7 +51,6 @@ struct sodecl_num {
     __device__ __forceinline__ sodecl_num &operator+=(sodecl_num o) { v = v + o.v; return *this; }
     __device__ __forceinline__ sodecl_num &operator-=(sodecl_num o) { v = v - o.v; return *this; }
     __device__ __forceinline__ sodecl_num &operator*=(sodecl_num o) { v = v * o.v; return *this; }
-    __device__ __forceinline__ sodecl_num &operator/=(sodecl_num o) { v = sodecl_div_rcp(v, o.v); return *this; }
     __device__ __forceinline__ sodecl_num &operator++() { v = v + (sodecl_num_t)1; return *this; }
     __device__ __forceinline__ sodecl_num &operator--() { v = v - (sodecl_num_t)1; return *this; }
 };
@@ -57,13 +59,16 @@ __device__ __forceinline__ sodecl_num operator-(sodecl_num a) { return sodecl_nu
 __device__ __forceinline__ sodecl_num operator+(sodecl_num a, sodecl_num b) { return sodecl_num(a.v + b.v); }
 __device__ __forceinline__ sodecl_num operator-(sodecl_num a, sodecl_num b) { return sodecl_num(a.v - b.v); }
 __device__ __forceinline__ sodecl_num operator*(sodecl_num a, sodecl_num b) { return sodecl_num(a.v * b.v); }
-__device__ __forceinline__ sodecl_num operator/(sodecl_num a, sodecl_num b) { return sodecl_num(sodecl_div_rcp(a.v, b.v)); }
 __device__ __forceinline__ bool operator<(sodecl_num a, sodecl_num b) { return a.v < b.v; }
 __device__ __forceinline__ bool operator>(sodecl_num a, sodecl_num b) { return a.v > b.v; }
 __device__ __forceinline__ bool operator<=(sodecl_num a, sodecl_num b) { return a.v <= b.v; }
 __device__ __forceinline__ bool operator>=(sodecl_num a, sodecl_num b) { return a.v >= b.v; }
 __device__ __forceinline__ bool operator==(sodecl_num a, sodecl_num b) { return a.v == b.v; }
 __device__ __forceinline__ bool operator!=(sodecl_num a, sodecl_num b) { return a.v != b.v; }
+}  // namespace sodecl_numeric
+using sodecl_numeric::sodecl_num;
+__device__ __forceinline__ sodecl_num operator/(sodecl_num a, sodecl_num b) { return sodecl_num(sodecl_div_rcp(a.v, b.v)); }
+__device__ __forceinline__ sodecl_num &operator/=(sodecl_num &a, sodecl_num b) { return a = a / b; }
 #define SODECL_NUM_UNARY(fn) \
     __device__ __forceinline__ sodecl_num fn(sodecl_num a) { return sodecl_num(::fn(a.v)); }
 SODECL_NUM_UNARY(exp) SODECL_NUM_UNARY(exp2) SODECL_NUM_UNARY(expm1) SODECL_NUM_UNARY(log)
@@ -89,13 +94,28 @@ __device__ __forceinline__ bool signbit(sodecl_num a) { return ::signbit(a.v); }
 __device__ __forceinline__ void sincos(sodecl_num a, sodecl_num *s, sodecl_num *c) { ::sincos(a.v, &s->v, &c->v); }
 #endif
 
+#if SODECL_FP32
+typedef float sodecl_scalar_t;
+#else
+typedef double sodecl_scalar_t;
+#endif
 #if SODECL_FAST_DIV
 typedef sodecl_num real_t;
-#elif SODECL_FP32
-typedef float real_t;
 #else
-typedef double real_t;
+typedef sodecl_scalar_t real_t;
 #endif
+
+// lanes per orbit: a group's shared vectors, and one lane's place in the group
+// (solvers.cuh)
+struct sodecl_lanes_view {
+    real_t *Y;       // state
+    real_t *A, *B;   // RK4: probes; Newton: iterate x, midpoint
+    real_t *D, *UP, *LO, *V, *DX;  // Newton: the banded system and its solution
+    real_t *P;       // parameters
+    real_t *NZ;      // noise of the step
+    int lane;        // lane within the group
+    unsigned mask;   // lanes taking part in the group's barriers and shuffles
+};
 
 // OpenCL C qualifiers: no meaning for a per-thread device function
 #define __kernel

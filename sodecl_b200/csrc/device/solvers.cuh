@@ -30,6 +30,11 @@
 //   SODECL_HAS_ROW_BAND  the system file defines sode_system_row_band
 //   SODECL_PAIR_STORES   one-thread kernel: records written two orbits per
 //                        vector store (sodecl_store_pairs)
+//   SODECL_SPECULATE     explicit and stochastic solvers: steps run on the
+//                        speculative copy of the system file (fastmath.cuh),
+//                        which with this file's step functions lies in
+//                        namespace sodecl_spec (SODECL_SPEC_COPY, assembled
+//                        first)
 
 #ifndef SODECL_MIN_BLOCKS
 #define SODECL_MIN_BLOCKS 1
@@ -43,6 +48,16 @@ template <> struct sodecl_pair_of<float> { typedef float2 type; };
 #ifndef SODECL_PAIR_STORES
 #define SODECL_PAIR_STORES 0
 #endif
+#ifndef SODECL_SPECULATE
+#define SODECL_SPECULATE 0
+#endif
+// Steps between two looks at a thread's flag.  A look costs a shared-memory
+// load and a branch on the step's chain, and a copy of the state before it; a
+// flag repeats the whole run.  (Oculomotor RK4 where nearly every orbit
+// diverges, 2^18 orbits x 1000 steps of dt 1e-3: 7.6 ms with 8, 8.0 with 16,
+// 11.8 with 64; at a stable step the three are within 1 %.)
+#undef SODECL_SPEC_RUN
+#define SODECL_SPEC_RUN 8
 #if SODECL_PAIR_STORES && (SODECL_LANES != 1 || SODECL_SOLVER > 2)
 #error "paired record stores serve the one-thread kernel of the explicit and stochastic solvers"
 #endif
@@ -297,8 +312,8 @@ __device__ __forceinline__ void sodecl_draw_noise(sodecl_i64 gid, double &counte
         sodecl_u64 w0, w1;
         sodecl_threefry2x64_20((sodecl_u64)gid, sodecl_counter_word(counter), SODECL_TF_KEY0, SODECL_TF_KEY1, w0, w1);
         counter = counter + 1;
-        real_t n0, n1;
-        sodecl_gaussian_pair<real_t>(w0, w1, sqrt_h, n0, n1);
+        sodecl_scalar_t n0, n1;
+        sodecl_gaussian_pair<sodecl_scalar_t>(w0, w1, (sodecl_scalar_t)sqrt_h, n0, n1);
         noise[2 * c] = n0;
         if (2 * c + 1 < _numnoi_)
             noise[2 * c + 1] = n1;
@@ -471,6 +486,44 @@ __device__ __forceinline__ void sodecl_advance(real_t &t, real_t *y, real_t *p, 
     for (int e = 0; e < _numeq_; ++e) y[e] = ynew[e];
 }
 
+#ifndef SODECL_SPEC_COPY
+// m steps of the configured solver (m at most SODECL_SPEC_RUN in speculative
+// programs).
+__device__ __forceinline__ void sodecl_advance_run(real_t &t, real_t *y, real_t *p, sodecl_i64 gid, double &counter,
+                                                   sodecl_i64 &passes, int &capped, int m)
+{
+#if SODECL_SPECULATE && SODECL_LANES == 1
+    const real_t t0 = t;
+    const double counter0 = counter;
+    real_t y0[_numeq_];
+#pragma unroll SODECL_EQ_UNROLL
+    for (int e = 0; e < _numeq_; ++e) y0[e] = y[e];
+#pragma unroll 1
+    for (int q = 0; q < m; ++q) sodecl_spec::sodecl_advance(t, y, p, gid, counter, passes, capped);
+    if (sodecl_raised()) {
+        sodecl_lower();
+        bool diverged = true;
+#pragma unroll SODECL_EQ_UNROLL
+        for (int e = 0; e < _numeq_; ++e) diverged = diverged && y0[e] != y0[e];
+        if (!diverged) {
+            // (as a function of its own this cost the step loop more registers
+            // and spills: oculomotor RK4, 2^18 orbits x 1000 steps, 5.72
+            // against 5.67 ms, and 7.5 against 6.6 ms at dt 1e-3)
+            real_t tc = t0;
+            double cc = counter0;
+#pragma unroll SODECL_EQ_UNROLL
+            for (int e = 0; e < _numeq_; ++e) y[e] = y0[e];
+#pragma unroll 1
+            for (int q = 0; q < m; ++q) sodecl_advance(tc, y, p, gid, cc, passes, capped);
+        }
+    }
+#else
+#pragma unroll 1
+    for (int q = 0; q < m; ++q) sodecl_advance(t, y, p, gid, counter, passes, capped);
+#endif
+}
+#endif  // SODECL_SPEC_COPY
+
 #if SODECL_LANES > 1
 // ---------------------------------------------------------------------------
 // Lanes per orbit, for wide systems.  With one thread per orbit, a system of
@@ -522,16 +575,6 @@ __device__ __forceinline__ void sodecl_advance(real_t &t, real_t *y, real_t *p, 
 #endif
 #define SODECL_SLOT_RAW (SODECL_LANES_NVEC * (_numeq_) + (_numpar_) + (_numnoi_))
 #define SODECL_SLOT ((SODECL_SLOT_RAW) | 1)
-
-struct sodecl_lanes_view {
-    real_t *Y;       // state
-    real_t *A, *B;   // RK4: probes; Newton: iterate x, midpoint
-    real_t *D, *UP, *LO, *V, *DX;  // Newton: the banded system and its solution
-    real_t *P;       // parameters
-    real_t *NZ;      // noise of the step
-    int lane;        // lane within the group
-    unsigned mask;   // lanes taking part in the group's barriers and shuffles
-};
 
 __device__ __forceinline__ sodecl_lanes_view sodecl_lanes_slot(real_t *slot, int lane, unsigned mask)
 {
@@ -789,8 +832,8 @@ __device__ __forceinline__ void sodecl_lanes_advance(real_t &t, real_t *yown, co
         sodecl_u64 w0, w1;
         sodecl_threefry2x64_20((sodecl_u64)gid, sodecl_counter_word(sodecl_counter_plus(counter, c)), SODECL_TF_KEY0,
                                SODECL_TF_KEY1, w0, w1);
-        real_t n0, n1;
-        sodecl_gaussian_pair<real_t>(w0, w1, sqrt_h, n0, n1);
+        sodecl_scalar_t n0, n1;
+        sodecl_gaussian_pair<sodecl_scalar_t>(w0, w1, (sodecl_scalar_t)sqrt_h, n0, n1);
         v.NZ[2 * c] = n0;
         if (2 * c + 1 < _numnoi_) v.NZ[2 * c + 1] = n1;
     }
@@ -823,6 +866,50 @@ __device__ __forceinline__ void sodecl_lanes_advance(real_t &t, real_t *yown, co
     }
     __syncwarp(v.mask);
 }
+
+#ifndef SODECL_SPEC_COPY
+// m steps of the configured solver (m at most SODECL_SPEC_RUN in speculative
+// programs), by every lane of the group together.
+__device__ __forceinline__ void sodecl_lanes_advance_run(real_t &t, real_t *yown, const sodecl_lanes_view &v,
+                                                         sodecl_i64 gid, double &counter, sodecl_i64 &passes,
+                                                         int &capped, int m)
+{
+#if SODECL_SPECULATE
+    const real_t t0 = t;
+    const double counter0 = counter;
+    real_t y0[SODECL_ROWS];
+#pragma unroll
+    for (int k = 0; k < SODECL_ROWS; ++k) y0[k] = yown[k];
+#pragma unroll 1
+    for (int q = 0; q < m; ++q) sodecl_spec::sodecl_lanes_advance(t, yown, v, gid, counter, passes, capped);
+    // one lane's flag spoils every row of the orbit, so the group repeats the
+    // run as one (the ballots' bits of other groups, if any, do not count)
+    if (__ballot_sync(v.mask, sodecl_raised()) & v.mask) {
+        sodecl_lower();
+        bool finite = false;
+#pragma unroll
+        for (int k = 0; k < SODECL_ROWS; ++k)
+            finite = finite || (v.lane + k * SODECL_LANES < _numeq_ && y0[k] == y0[k]);
+        if (__ballot_sync(v.mask, finite) & v.mask) {
+            real_t tc = t0;
+            double cc = counter0;
+#pragma unroll
+            for (int k = 0; k < SODECL_ROWS; ++k) {
+                const int r = v.lane + k * SODECL_LANES;
+                yown[k] = y0[k];
+                if (r < _numeq_) v.Y[r] = y0[k];
+            }
+            __syncwarp(v.mask);
+#pragma unroll 1
+            for (int q = 0; q < m; ++q) sodecl_lanes_advance(tc, yown, v, gid, cc, passes, capped);
+        }
+    }
+#else
+#pragma unroll 1
+    for (int q = 0; q < m; ++q) sodecl_lanes_advance(t, yown, v, gid, counter, passes, capped);
+#endif
+}
+#endif  // SODECL_SPEC_COPY
 #endif  // SODECL_LANES > 1
 
 #ifndef SODECL_STEPS_ONLY
@@ -1089,6 +1176,9 @@ sodecl_orbits(const sodecl_args a)
     const sodecl_i64 i = (sodecl_i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n)
         return;
+#if SODECL_SPECULATE
+    sodecl_lower();
+#endif
 
     real_t y[_numeq_];
     real_t p[SODECL_NPAR_ALLOC];
@@ -1111,9 +1201,13 @@ sodecl_orbits(const sodecl_args a)
     for (int c = a.chunk_begin; c < a.chunk_end; ++c) {
         if (a.records)
             sodecl_store_record(a, c, i, y, flags);
+#if SODECL_SPECULATE
 #pragma unroll 1
-        for (int s = 0; s < _numsteps_; ++s)
-            sodecl_advance(t, y, p, gid, counter, passes, capped);
+        for (int left = _numsteps_; left > 0; left -= SODECL_SPEC_RUN)
+            sodecl_advance_run(t, y, p, gid, counter, passes, capped, min(SODECL_SPEC_RUN, left));
+#else
+        sodecl_advance_run(t, y, p, gid, counter, passes, capped, _numsteps_);
+#endif
     }
     sodecl_orbit_out(a, i, t, y, counter, passes, capped, flags);
 }
@@ -1142,6 +1236,9 @@ extern "C" __global__ void __launch_bounds__(SODECL_BLOCK_MAX, SODECL_MIN_BLOCKS
 sodecl_orbits(const sodecl_args a)
 {
     extern __shared__ __align__(16) unsigned char sodecl_smem[];
+#if SODECL_SPECULATE
+    sodecl_lower();
+#endif
     const int lane = threadIdx.x % SODECL_LANES;
     // the group's own lanes: groups of a warp leave a Newton iteration after
     // different numbers of passes, so no barrier or shuffle names another group
@@ -1178,9 +1275,13 @@ sodecl_orbits(const sodecl_args a)
 #pragma unroll 1
     for (int c = a.chunk_begin; c < a.chunk_end; ++c) {
         if (a.records && live) sodecl_lanes_store(a, c, i, yown, lane, flags);
+#if SODECL_SPECULATE
 #pragma unroll 1
-        for (int s = 0; s < _numsteps_; ++s)
-            sodecl_lanes_advance(t, yown, v, gid, counter, passes, capped);
+        for (int left = _numsteps_; left > 0; left -= SODECL_SPEC_RUN)
+            sodecl_lanes_advance_run(t, yown, v, gid, counter, passes, capped, min(SODECL_SPEC_RUN, left));
+#else
+        sodecl_lanes_advance_run(t, yown, v, gid, counter, passes, capped, _numsteps_);
+#endif
     }
     if (a.write_final && a.records && live) sodecl_lanes_store(a, a.chunk_end, i, yown, lane, flags);
 

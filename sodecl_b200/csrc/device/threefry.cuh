@@ -65,7 +65,20 @@ __device__ __forceinline__ unsigned long long sodecl_counter_word(double c)
     return (unsigned long long)(long long)c;
 }
 
-// One draw's two words -> a Box-Muller pair scaled by sqrt(h), in precision R:
+// The functions of the pair below: in FP64 straight-line code (mathcore.cuh;
+// their arguments lie inside its ranges), so that the draws of a step overlap;
+// in FP32 the library's.
+__device__ __forceinline__ double sodecl_noise_log(double x) { return sodecl_log_core(x); }
+__device__ __forceinline__ double sodecl_noise_sqrt(double x) { return sodecl_sqrt_core(x); }
+__device__ __forceinline__ double sodecl_noise_sin(double x) { return sodecl_sin_core(x); }
+__device__ __forceinline__ double sodecl_noise_cos(double x) { return sodecl_cos_core(x); }
+__device__ __forceinline__ float sodecl_noise_log(float x) { return log(x); }
+__device__ __forceinline__ float sodecl_noise_sqrt(float x) { return sqrt(x); }
+__device__ __forceinline__ float sodecl_noise_sin(float x) { return sin(x); }
+__device__ __forceinline__ float sodecl_noise_cos(float x) { return cos(x); }
+
+// One draw's two words -> a Box-Muller pair scaled by sqrt(h), in precision R
+// (double or float):
 //   n0 = sqrt(-2 ln u0) cos(2 pi u1) sqrt(h),  n1 = ... sin(...)
 // (stochastic_solver_caller.cl:56-63).
 template <class R>
@@ -73,10 +86,10 @@ __device__ __forceinline__ void sodecl_gaussian_pair(unsigned long long w0, unsi
 {
     const R u0 = (R)sodecl_u01_open_open(w0);
     const R u1 = (R)sodecl_u01_open_open(w1);
-    const R rad = sqrt((R)(-2) * log(u0));
+    const R rad = sodecl_noise_sqrt((R)(-2) * sodecl_noise_log(u0));
     const R ang = (R)(2 * 3.14159265358979323846) * u1;
-    n0 = (rad * cos(ang)) * sqrt_h;
-    n1 = (rad * sin(ang)) * sqrt_h;
+    n0 = (rad * sodecl_noise_cos(ang)) * sqrt_h;
+    n1 = (rad * sodecl_noise_sin(ang)) * sqrt_h;
 }
 
 #endif

@@ -31,7 +31,7 @@
 namespace sodecl_b200 {
 
 namespace {
-#include "embedded_sources.inc"  // kFastDivSrc kPreludeSrc kThreefrySrc kSolversSrc kBatchSrc kAdjointSrc (build.py)
+#include "embedded_sources.inc"  // kFastDivSrc kPreludeSrc kMathCoreSrc kFastMathSrc kThreefrySrc kSolversSrc kBatchSrc kAdjointSrc (build.py)
 
 // Splits `src` into code / comment / literal runs and passes the code runs
 // through `on_code`; comments are kept (or blanked), literals kept.
@@ -377,6 +377,8 @@ SystemTraits inspect_system(const std::string &src)
     t.has_row_band = defines_function(stripped, "sode_system_row_band");
     t.has_vjp = defines_function(stripped, "calc_vjp");
     t.uses_listsize = std::regex_search(stripped, std::regex("\\b_listsize_\\b"));
+    t.uses_division = stripped.find('/') != std::string::npos;
+    t.uses_math = std::regex_search(stripped, std::regex("\\b(native_|half_)?(sin|cos|sincos|exp)\\s*\\("));
     return t;
 }
 
@@ -385,6 +387,74 @@ int lanes_slot_words(const ProgramSpec &spec)
     const int nvec = spec.solver == 2 ? 3 : (spec.solver == 3 || spec.solver == 4) ? 8 : 1;
     return (nvec * spec.num_equat + spec.num_params + spec.num_noi) | 1;
 }
+
+namespace {
+
+// Names of the object-like and function-like macros a source #defines, so a
+// batch program can #undef them after each class.
+std::vector<std::string> defined_macros(const std::string &src)
+{
+    std::vector<std::string> names;
+    const std::regex def("^[ \\t]*#[ \\t]*define[ \\t]+([A-Za-z_][A-Za-z0-9_]*)");
+    const std::string stripped = scan_code(src, [](const std::string &x) { return x; }, false);
+    for (std::sregex_iterator it(stripped.begin(), stripped.end(), def), end; it != end; ++it)
+        names.push_back((*it)[1].str());
+    return names;
+}
+
+// The functions of device/fastmath.cuh in place of the library's, for the
+// copy of the system file that follows: copy is "spec" (the speculative copy)
+// or "full" (the plain one).  The stochastic solver takes the finer exp: beside
+// a step's noise (a logarithm, a root and a sine pair for every two processes)
+// its six instructions are few, where they cost RK4 a tenth.
+std::string math_macros(const std::string &copy, int solver)
+{
+    std::string s;
+    for (const std::string fn : {"sin", "cos", "exp", "sincos"})
+        s += "#define " + fn + "(...) sodecl_" + copy + "_" + fn + (fn == "exp" && solver == 0 ? "_fine" : "") +
+             "(__VA_ARGS__)\n";
+    return s;
+}
+
+std::string undef_math_macros() { return "#undef sin\n#undef cos\n#undef exp\n#undef sincos\n"; }
+
+std::string undef_lines(const std::vector<std::string> &names)
+{
+    std::string s;
+    for (const auto &n : names) s += "#undef " + n + "\n";
+    return s;
+}
+
+// The system file as the solvers see it: with speculative steps its
+// speculative copy first, which with the solvers' step functions lies in a
+// namespace of its own, then the plain copy.
+std::string user_text(const std::string &src, const std::string &name, const std::string &as_double, bool speculate,
+                      int solver)
+{
+    const std::string plain = (as_double.empty() ? "" : "#undef double\n");
+    const std::string user = "#line 1 \"" + name + "\"\n" + src + "\n";
+    if (!speculate) return as_double + user + plain;
+    return "namespace sodecl_spec {\nSODECL_SPEC_QUOTIENT\n" + as_double + math_macros("spec", solver) + user +
+           undef_math_macros() + plain + undef_lines(defined_macros(src)) +
+           "#ifndef SODECL_STEPS_ONLY\n#define SODECL_STEPS_ONLY 1\n#define SODECL_STEPS_ONLY_HERE 1\n#endif\n"
+           "#define SODECL_SPEC_COPY 1\n#line 1 \"solvers.cuh\"\n" + kSolversSrc +
+           "\n#undef SODECL_SPEC_COPY\n#ifdef SODECL_STEPS_ONLY_HERE\n#undef SODECL_STEPS_ONLY_HERE\n"
+           "#undef SODECL_STEPS_ONLY\n#endif\n}  // namespace sodecl_spec\n" +
+           as_double + math_macros("full", solver) + user + undef_math_macros() + plain;
+}
+
+// Whether speculative steps have something to gain: a function of
+// device/fastmath.cuh or a reciprocal quotient (RK4 divides by itself) in a
+// solver whose step is a fixed sequence of evaluations.  A repeated step would
+// print twice.  One thread's arrays of more than 256 equations fill its local
+// memory already; the copy of the state would only add to it.
+bool worth_speculating(const ProgramSpec &s, const SystemTraits &t, const std::string &src)
+{
+    return s.speculate && src.find("printf") == std::string::npos && (s.lanes > 1 || s.num_equat <= 256) &&
+           (t.uses_math || (s.fast_div && (t.uses_division || s.solver == 2)));
+}
+
+}  // namespace
 
 std::string assemble(const ProgramSpec &spec, const std::string &system_src, const SystemTraits &traits)
 {
@@ -405,7 +475,10 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
     s << "#define SODECL_HAS_STOCH_ROW " << (traits.has_stoch_row ? 1 : 0) << "\n";
     s << "#define SODECL_HAS_JAC_BAND " << (traits.has_jac_band ? 1 : 0) << "\n";
     s << "#define SODECL_HAS_ROW_BAND " << (traits.has_row_band ? 1 : 0) << "\n";
-    s << kFastDivSrc << "\n" << kPreludeSrc << "\n" << kThreefrySrc << "\n";
+    s << "#define SODECL_SPECULATE " << (spec.speculate ? 1 : 0) << "\n";
+    s << kFastDivSrc << "\n" << kPreludeSrc << "\n" << kMathCoreSrc << "\n";
+    if (spec.speculate) s << kFastMathSrc << "\n";
+    s << kThreefrySrc << "\n";
     // the reference's program defines (src/sodeclmgr.cpp:379-430); _listsize_
     // only when the system file names it, so one program serves every size
     s << "#define _numnoi_ " << spec.num_noi << "\n";
@@ -426,21 +499,21 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
         std::snprintf(buf, sizeof buf, "#define SODECL_RTOL %a\n#define SODECL_ATOL %a\n", spec.rtol, spec.atol);
         s << buf << "#define SODECL_MAX_STEPS " << spec.max_steps << "\n";
     }
-    if (spec.fast_div) s << "#define double sodecl_num\n";
-    else if (spec.fp32) s << "#define double float\n";
-    s << "#line 1 \"system.cl\"\n";
-    const std::string user = relax_parameter_bounds(system_src);
-    s << (spec.fp32 ? suffix_float_literals(user) : user) << "\n";
-    if (spec.fp32 || spec.fast_div) s << "#undef double\n";
+    const std::string as_double = spec.fast_div ? "#define double sodecl_num\n" : spec.fp32 ? "#define double float\n" : "";
+    const std::string bounded = relax_parameter_bounds(system_src);
+    s << user_text(spec.fp32 ? suffix_float_literals(bounded) : bounded, "system.cl", as_double, spec.speculate,
+                   spec.solver);
     s << "#line 1 \"solvers.cuh\"\n" << kSolversSrc << "\n";
     return s.str();
 }
 
 namespace {
 
-std::shared_ptr<const Program> compile_text(std::string source, bool fmad, bool fast_div, const char *kernel)
+std::shared_ptr<const Program> compile_text(std::string source, bool fmad, bool fast_div, const char *kernel,
+                                            bool speculate = false)
 {
     auto prog = std::make_shared<Program>();
+    prog->speculate = speculate;
     prog->source = std::move(source);
     prog->fast_div = fast_div;
     prog->kernel_name = kernel;
@@ -501,19 +574,7 @@ std::shared_ptr<const Program> compile_text(std::string source, bool fmad, bool 
 std::shared_ptr<const Program> compile_one(const ProgramSpec &spec, const std::string &system_src,
                                            const SystemTraits &traits)
 {
-    return compile_text(assemble(spec, system_src, traits), spec.fmad, spec.fast_div, "sodecl_orbits");
-}
-
-// Names of the object-like and function-like macros a source #defines, so a
-// batch program can #undef them after each class.
-std::vector<std::string> defined_macros(const std::string &src)
-{
-    std::vector<std::string> names;
-    const std::regex def("^[ \\t]*#[ \\t]*define[ \\t]+([A-Za-z_][A-Za-z0-9_]*)");
-    const std::string stripped = scan_code(src, [](const std::string &x) { return x; }, false);
-    for (std::sregex_iterator it(stripped.begin(), stripped.end(), def), end; it != end; ++it)
-        names.push_back((*it)[1].str());
-    return names;
+    return compile_text(assemble(spec, system_src, traits), spec.fmad, spec.fast_div, "sodecl_orbits", spec.speculate);
 }
 
 }  // namespace
@@ -528,7 +589,8 @@ int batch_warp_words(const std::vector<BatchClass> &classes)
 
 namespace {
 
-std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div, int block_max, int min_blocks)
+std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div, bool speculate, int block_max,
+                           int min_blocks)
 {
     std::ostringstream s;
     s << "// SODECL batch program generated by libsodecl_cuda (sm_100a)\n";
@@ -536,16 +598,22 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
     s << "#define SODECL_FAST_DIV " << (fast_div ? 1 : 0) << "\n";
     s << "#define SODECL_BLOCK_MAX " << block_max << "\n";
     s << "#define SODECL_BATCH_MIN_BLOCKS " << std::max(1, min_blocks) << "\n";
-    s << kFastDivSrc << "\n" << kPreludeSrc << "\n" << kThreefrySrc << "\n" << kBatchSrc << "\n";
+    s << kFastDivSrc << "\n" << kPreludeSrc << "\n" << kMathCoreSrc << "\n";
+    if (speculate) s << kFastMathSrc << "\n";
+    s << kThreefrySrc << "\n" << kBatchSrc << "\n";
     static const char *per_class[] = {"SODECL_SOLVER", "SODECL_HAS_JACOBIAN", "SODECL_HAS_STOCH", "SODECL_NEWTON_MAX",
                                       "_numnoi_", "_numsteps_", "_m_dt_", "_numeq_", "_numpar_", "_epsilon1_",
                                       "SODECL_L2_BOUND", "_listsize_", "SODECL_BATCH_CLASS_BODY", "SODECL_LANES",
                                       "SODECL_HAS_ROW", "SODECL_HAS_STOCH_ROW", "SODECL_HAS_JAC_BAND",
-                                      "SODECL_HAS_ROW_BAND"};
+                                      "SODECL_HAS_ROW_BAND", "SODECL_SPECULATE"};
     for (size_t k = 0; k < classes.size(); ++k) {
         const ProgramSpec &sp = classes[k].spec;
         const std::string &src = classes[k].system_src;
         const SystemTraits tr = inspect_system(src);
+        ProgramSpec gain = sp;
+        gain.fast_div = fast_div;
+        gain.speculate = speculate && sp.solver <= 2;
+        const bool spec = worth_speculating(gain, tr, src);
         s << "\n// ---- class " << k << "\n";
         for (const char *m : per_class) s << "#undef " << m << "\n";
         s << "#define SODECL_SOLVER " << sp.solver << "\n";
@@ -553,6 +621,7 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
         s << "#define SODECL_HAS_STOCH " << (tr.has_stoch ? 1 : 0) << "\n";
         s << "#define SODECL_NEWTON_MAX " << sp.newton_max_iter << "\n";
         s << "#define SODECL_LANES " << sp.lanes << "\n";
+        s << "#define SODECL_SPECULATE " << (spec ? 1 : 0) << "\n";
         s << "#define SODECL_HAS_ROW " << (tr.has_row ? 1 : 0) << "\n";
         s << "#define SODECL_HAS_STOCH_ROW " << (tr.has_stoch_row ? 1 : 0) << "\n";
         s << "#define SODECL_HAS_JAC_BAND " << (tr.has_jac_band ? 1 : 0) << "\n";
@@ -566,9 +635,8 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
         s << "#define _epsilon1_ " << print_like_reference(sp.newton_tol) << "\n";
         s << l2_bound_define(sp.newton_tol, false);
         s << "namespace sodecl_cls_" << k << " {\n";
-        if (fast_div) s << "#define double sodecl_num\n";
-        s << "#line 1 \"class" << k << ".cl\"\n" << relax_parameter_bounds(src) << "\n";
-        if (fast_div) s << "#undef double\n";
+        s << user_text(relax_parameter_bounds(src), "class" + std::to_string(k) + ".cl",
+                       fast_div ? "#define double sodecl_num\n" : "", spec, sp.solver);
         for (const auto &m : defined_macros(src)) s << "#undef " << m << "\n";
         s << "#line 1 \"solvers.cuh\"\n" << kSolversSrc << "\n";
         s << "#define SODECL_BATCH_CLASS_BODY 1\n#line 1 \"batch.cuh\"\n" << kBatchSrc << "\n";
@@ -585,6 +653,7 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
     } else {
         s << "    double *warp_smem = nullptr;\n";
     }
+    if (speculate) s << "    sodecl_lower();\n";
     s << "    for (int k = 0; k < a.nclasses; ++k) {\n        switch (a.order[k]) {\n";
     for (size_t k = 0; k < classes.size(); ++k)
         s << "        case " << k << ": sodecl_cls_" << k << "::sodecl_class_run(a, " << k << ", warp_smem); break;\n";
@@ -609,7 +678,7 @@ std::string assemble_adjoint(const ProgramSpec &spec, const std::string &src, in
     s << "#define SODECL_TAPE_CAP " << tape_cap << "\n";
     s << "#define SODECL_ADJ_MODE " << mode << "\n";
     s << "#define SODECL_ADJ_GRADIENT " << (gradient ? 1 : 0) << "\n";
-    s << kFastDivSrc << "\n" << kPreludeSrc << "\n" << kThreefrySrc << "\n" << kAdjointSrc << "\n";
+    s << kFastDivSrc << "\n" << kPreludeSrc << "\n" << kMathCoreSrc << "\n" << kThreefrySrc << "\n" << kAdjointSrc << "\n";
     s << "#define _numnoi_ " << spec.num_noi << "\n";
     s << "#define _listsize_ " << spec.list_size << "\n";
     s << "#define _numsteps_ " << spec.kernel_steps << "\n";
@@ -657,13 +726,19 @@ std::shared_ptr<const Program> build_batch(const std::vector<BatchClass> &classe
     bool fd = fast_div;
     for (const auto &c : classes)
         if (c.system_src.find("printf") != std::string::npos) fd = false;
-    if (fd) {
-        try {
-            return compile_text(assemble_batch(classes, true, block_max, min_blocks), fmad, true, "sodecl_batch");
-        } catch (const std::exception &) {
+    // as for one system: the plainer programs where a system file needs them
+    for (const bool div : {true, false}) {
+        for (const bool speculate : {true, false}) {
+            if (div && !fd) continue;
+            const std::string text = assemble_batch(classes, div, speculate, block_max, min_blocks);
+            if (!div && !speculate) return compile_text(text, fmad, div, "sodecl_batch");
+            try {
+                return compile_text(text, fmad, div, "sodecl_batch", speculate);
+            } catch (const std::exception &) {
+            }
         }
     }
-    return compile_text(assemble_batch(classes, false, block_max, min_blocks), fmad, false, "sodecl_batch");
+    return nullptr;  // not reached
 }
 
 std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string &system_src)
@@ -671,15 +746,26 @@ std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string 
     const SystemTraits traits = inspect_system(system_src);
     ProgramSpec s = spec;
     // the wrapper type would hand a struct to printf's varargs
-    if (s.fast_div && system_src.find("printf") != std::string::npos) s.fast_div = false;
-    if (!s.fast_div) return compile_one(s, system_src, traits);
-    try {
-        return compile_one(s, system_src, traits);
-    } catch (const std::exception &) {
-        // the system file needs plain `double` (an implicit conversion, say)
-        s.fast_div = false;
-        return compile_one(s, system_src, traits);
+    if (system_src.find("printf") != std::string::npos) s.fast_div = false;
+    s.speculate = worth_speculating(s, traits, system_src);
+    // a system file that needs plain `double` (an implicit conversion, say)
+    // does not compile with the wrapper, and one that declares or redefines
+    // the math functions does not with fastmath.cuh's: the next plainer
+    // program is built instead, the division mode kept as long as it can be
+    for (const bool fast_div : {true, false}) {
+        for (const bool speculate : {true, false}) {
+            if ((fast_div && !s.fast_div) || (speculate && !s.speculate)) continue;
+            ProgramSpec t = s;
+            t.fast_div = fast_div;
+            t.speculate = speculate;
+            if (!fast_div && !speculate) return compile_one(t, system_src, traits);
+            try {
+                return compile_one(t, system_src, traits);
+            } catch (const std::exception &) {
+            }
+        }
     }
+    return nullptr;  // not reached
 }
 
 }  // namespace sodecl_b200

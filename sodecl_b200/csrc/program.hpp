@@ -25,6 +25,7 @@ struct ProgramSpec {
     int block_max = 256;
     int min_blocks = 0;
     int lanes = 1;           // lanes per orbit (1, or a power of two up to 32)
+    bool speculate = false;  // steps on the speculative copy of the system file (device/fastmath.cuh)
     bool pair_stores = false;  // one thread per orbit: records two orbits per vector store
     double rtol = 1e-6;      // adaptive solver (solver 5): error tolerances and
     double atol = 1e-9;      // step attempts per record interval
@@ -37,6 +38,7 @@ struct Program {
     std::vector<char> cubin;
     std::string kernel_name = "sodecl_orbits";
     bool fast_div = false;   // built with the reciprocal-division wrapper
+    bool speculate = false;  // built with speculative steps (their flags take static shared memory)
 };
 
 // What the system file provides.
@@ -51,6 +53,8 @@ struct SystemTraits {
     bool has_row_band = false;   // sode_system_row_band (a row's right-hand side and band together)
     bool has_vjp = false;        // calc_vjp (v^T df/dy and v^T df/dp), used by the adjoint
     bool uses_listsize = false;
+    bool uses_division = false;
+    bool uses_math = false;      // calls sin, cos, sincos or exp (the functions of device/fastmath.cuh)
 };
 
 SystemTraits inspect_system(const std::string &src);

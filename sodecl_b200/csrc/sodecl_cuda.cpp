@@ -288,6 +288,20 @@ void free_buffers(sodecl_ctx *ctx)
     ctx->uploaded = false;
 }
 
+// The dynamic shared memory cap of one block of the lanes-per-orbit kernel.
+constexpr size_t kLanesSharedCap = 48 * 1024;
+
+// Speculative programs keep their threads' flags in static shared memory, so
+// a launch at the cap goes past the 48 KiB a block gets without asking.
+cudaError_t allow_dynamic_shared(const Program &prog, cudaKernel_t kernel, int lanes)
+{
+    if (!prog.speculate || lanes <= 1) return cudaSuccess;
+    return cudaFuncSetAttribute(reinterpret_cast<const void *>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(kLanesSharedCap));
+}
+
+int lanes_of(const sodecl_cfg &c) { return c.lanes_per_orbit > 1 ? c.lanes_per_orbit : 1; }
+
 // Loads the compiled program on the context's device and makes its streams.
 int ensure_gpu(sodecl_ctx *ctx)
 {
@@ -303,14 +317,13 @@ int ensure_gpu(sodecl_ctx *ctx)
     if (ctx->gpu_ready) return SODECL_OK;
     SODECL_CUDA_TRY(ctx, cudaLibraryLoadData(&ctx->lib, ctx->prog->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
     SODECL_CUDA_TRY(ctx, cudaLibraryGetKernel(&ctx->kernel, ctx->lib, ctx->prog->kernel_name.c_str()));
+    SODECL_CUDA_TRY(ctx, allow_dynamic_shared(*ctx->prog, ctx->kernel, lanes_of(ctx->cfg)));
     if (!ctx->stream) SODECL_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     if (!ctx->copy_stream) SODECL_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
     ctx->loaded_device = ctx->cfg.device;
     ctx->gpu_ready = true;
     return SODECL_OK;
 }
-
-int lanes_of(const sodecl_cfg &c) { return c.lanes_per_orbit > 1 ? c.lanes_per_orbit : 1; }
 
 // A piece of the record buffer: `count` doubles at element offset `off`,
 // ready once launch group `group` has finished.
@@ -403,10 +416,6 @@ bool lanes_supported(const sodecl_b200::SystemTraits &t, int solver)
     if (solver == SODECL_IMPLICIT_EULER || solver == SODECL_IMPLICIT_MIDPOINT) return t.has_jac_band;
     return true;
 }
-
-// Shared memory cap of one block of the lanes-per-orbit kernel (the default
-// dynamic shared memory limit, no opt-in needed).
-constexpr size_t kLanesSharedCap = 48 * 1024;
 
 // Launch geometry of the configured kernel for n orbits: threads per block,
 // blocks, dynamic shared memory.  One thread per orbit: the block size as
@@ -533,6 +542,12 @@ ProgramSpec make_spec(const sodecl_cfg &c)
         spec.min_blocks = std::max(1, 65536 / (spec.block_max * 85));
     spec.fast_div = reciprocal_division(c);
     spec.lanes = lanes_of(c);
+    // sin, cos and exp without branches (device/fastmath.cuh) in FP64 for the
+    // solvers whose step is a fixed sequence of evaluations.  The implicit and
+    // adaptive solvers decide by a tolerance how often they evaluate, so they
+    // keep the library's functions, and with them their pass and step counts
+    spec.speculate = !spec.fp32 && (c.solver == SODECL_EULER || c.solver == SODECL_RUNGE_KUTTA ||
+                                    c.solver == SODECL_STOCHASTIC_EULER);
     // paired stores need the pair's two threads at the same store with orbits
     // 2k and 2k+1: the one-thread kernel of the explicit and stochastic
     // solvers (the implicit and adaptive kernels store per lane, whenever that
@@ -1090,7 +1105,8 @@ int sodecl_cuda_autotune(sodecl_ctx *ctx, int64_t sample_orbits, int32_t sample_
         cudaLibrary_t lib = nullptr;
         cudaKernel_t kern = nullptr;
         if (cudaLibraryLoadData(&lib, prog->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) != cudaSuccess ||
-            cudaLibraryGetKernel(&kern, lib, prog->kernel_name.c_str()) != cudaSuccess) {
+            cudaLibraryGetKernel(&kern, lib, prog->kernel_name.c_str()) != cudaSuccess ||
+            allow_dynamic_shared(*prog, kern, c.lanes) != cudaSuccess) {
             cudaGetLastError();
             if (lib) cudaLibraryUnload(lib);
             return false;

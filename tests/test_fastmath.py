@@ -1,0 +1,108 @@
+"""The branch-free sin, cos, exp and quotient of the explicit and stochastic
+solvers (csrc/device/fastmath.cuh) at the edges of the ranges they cover, and
+the repetition of a run of steps that leaves them.
+
+Values: one Euler step of size 1 from y = -0 gives the right-hand side itself
+(-0 + f keeps f's sign of zero), compared with numpy.  Tolerances: sin, cos and
+exp are within 1.7, 1.7 and 0.9 ulp of the true value, CUDA's (outside the
+ranges) within 2, 2 and 1, numpy's within 1, so 3 ulp covers either; quotients
+are numpy's, bit for bit, but for results below 2^-960, which may be one ulp
+off."""
+import numpy as np
+import pytest
+
+from sodecl_b200 import Integrator
+
+pytestmark = pytest.mark.gpu
+
+VALUES = """
+void sode_system(double t, double y[_numeq_], double yout[_numeq_], double p[_numpar_])
+{
+	yout[0] = sin(p[0]);
+	yout[1] = cos(p[0]);
+	yout[2] = exp(p[0]);
+	yout[3] = p[0] / p[1];
+}
+"""
+# phases that grow past 2^30 in the middle of a run of steps
+DRIFT = """
+double sode_system_row(int i, double t, double y[_numeq_], double p[_numpar_])
+{
+	return p[0] + sin(y[i]) + cos(y[i]) / p[1];
+}
+void sode_system(double t, double y[_numeq_], double yout[_numeq_], double p[_numpar_])
+{
+	for (int i = 0; i < _numeq_; i++)
+	{
+		yout[i] = sode_system_row(i, t, y, p);
+	}
+}
+"""
+
+
+def edges():
+    pi = np.pi * np.arange(0, 9) / 4
+    lim = [2.0 ** 30, 708.0, 709.0, 709.78, 709.79, 745.0, 745.13, 746.0]
+    a = np.concatenate([[0.0, 1e-320, 1e-310, 5e-300, 1e-200, 1e-20, 1.0, 1e22, 1e200, 1.7e308, np.inf, np.nan], pi,
+                        np.nextafter(pi, 10), 1e6 + pi, lim, np.nextafter(lim, 0), np.nextafter(lim, 1e30)])
+    a = np.concatenate([a, -a])
+    b = np.array([1.0, 3.0, 6.0, 0.0045, 1e-30, 1e30, 2.0 ** -1000, np.nextafter(2.0 ** -1000, 0), 2.0 ** 960,
+                  np.nextafter(2.0 ** 960, 0), 1e-310, 1.7e308, 0.0, np.inf, np.nan])
+    b = np.concatenate([b, -b])
+    return np.repeat(a, b.size), np.tile(b, a.size)
+
+
+@pytest.mark.parametrize("fmad", [0, 1])
+def test_values_at_the_edges_of_the_ranges(fmad):
+    a, b = edges()
+    n = a.size
+    with Integrator(None, "euler", system_src=VALUES, dt=1.0, tspan=0.5, ksteps=1, neq=4, npar=2, orbits=n,
+                    fmad=bool(fmad)) as sim:
+        assert "#define SODECL_SPECULATE 1" in sim.program_source and sim.division == "reciprocal"
+        sim.upload(np.zeros(n), np.full((n, 4), -0.0), np.stack([a, b], axis=1))
+        got = sim.run()[1]
+    with np.errstate(all="ignore"):
+        want = np.stack([np.sin(a), np.cos(a), np.exp(a), a / b])
+        ulps = np.abs(got - want) / np.spacing(np.abs(want))
+    finite = np.isfinite(want)
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+    np.testing.assert_array_equal(got[~finite], want[~finite])
+
+    np.testing.assert_array_equal(np.signbit(got[~np.isnan(want)]), np.signbit(want[~np.isnan(want)]))
+    assert ulps[:3][finite[:3]].max() <= 3
+    q, w = got[3], want[3]
+    normal = finite[3] & ((np.abs(w) >= 2.0 ** -960) | (w == 0))
+    np.testing.assert_array_equal(q[normal], w[normal])
+    assert ulps[3][finite[3]].max() <= 1
+
+
+@pytest.mark.parametrize("ksteps", [1, 7, 8, 9, 40])
+@pytest.mark.parametrize("lanes", [1, 4])
+def test_runs_that_leave_the_range_are_repeated(ksteps, lanes):
+    """Orbits that stay inside, cross 2^30 early, late or start beyond, side by
+    side; each like alone, bit for bit, and like the same steps in numpy."""
+    n, neq, steps, h = 67, 5, 40, 0.01
+    rate = np.array([1.0, 1e10, 2e11, 3e9, 5e10])[np.arange(n) % 5]
+    y0 = np.linspace(0.0, 6.0, n * neq).reshape(n, neq) + np.where(np.arange(n) % 11 == 3, 2.0 ** 31, 0.0)[:, None]
+    p = np.stack([rate, np.full(n, 2.5)], axis=1)
+    kw = dict(system_src=DRIFT, dt=h, tspan=(steps - 0.5) * h, ksteps=ksteps, neq=neq, npar=2, lanes=lanes)
+
+    def run(sel):
+        with Integrator(None, "euler", orbits=len(sel), **kw) as sim:
+            sim.upload(np.zeros(len(sel)), y0[sel], p[sel])
+            return sim.run()
+
+    got = run(np.arange(n))
+    for sel in (np.array([1]), np.array([2, 3]), np.arange(5, 30, 5)):
+        np.testing.assert_array_equal(run(sel), got[:, :, sel])
+    y = y0.copy()
+    done = 0
+    for r in range(got.shape[0]):
+        # each step adds up to h (ulp of the sine + ...) and the rounding of y:
+        # a few ulps of the largest |y| a step, and the sine turns an error of
+        # y into one of h times it: exp(2 h steps) = 2.2 over the run
+        bound = 2.2 * (done + 1) * 4 * np.spacing(np.abs(y).max(axis=1))
+        assert np.all(np.abs(got[r].T - y) <= bound[:, None])
+        for _ in range(min(ksteps, got.shape[0] * ksteps)):
+            y = y + (p[:, :1] + np.sin(y) + np.cos(y) / 2.5) * h
+        done += ksteps
