@@ -1,5 +1,6 @@
 // sin, cos, exp and the quotient for the system files of the explicit and
-// stochastic solvers, without branches.
+// stochastic solvers, sin and cos for those of the implicit solvers, without
+// branches.
 //
 // The math library's functions end in a branch to a slow path for rare
 // arguments, and so does the reciprocal quotient, so the compiler cannot
@@ -16,7 +17,8 @@
 // same state (solvers.cuh).  Covered arguments give the same value in both
 // copies, so the result depends on the orbit's own state alone.  An orbit that
 // has diverged, every component NaN, stays so whatever its right-hand side
-// returns (y + ... is NaN), so its flag is ignored.
+// returns (y + ... is NaN), so its flag is ignored.  Programs without
+// speculative steps (the one-thread implicit kernel) use the plain copy alone.
 #ifndef SODECL_FASTMATH_CUH
 #define SODECL_FASTMATH_CUH
 

@@ -30,11 +30,11 @@
 //   SODECL_HAS_ROW_BAND  the system file defines sode_system_row_band
 //   SODECL_PAIR_STORES   one-thread kernel: records written two orbits per
 //                        vector store (sodecl_store_pairs)
-//   SODECL_SPECULATE     explicit and stochastic solvers: steps run on the
-//                        speculative copy of the system file (fastmath.cuh),
-//                        which with this file's step functions lies in
-//                        namespace sodecl_spec (SODECL_SPEC_COPY, assembled
-//                        first)
+//   SODECL_SPECULATE     explicit and stochastic solvers, implicit solvers with
+//                        lanes per orbit: steps run on the speculative copy
+//                        of the system file (fastmath.cuh), which with this
+//                        file's step functions lies in namespace sodecl_spec
+//                        (SODECL_SPEC_COPY, assembled first)
 
 #ifndef SODECL_MIN_BLOCKS
 #define SODECL_MIN_BLOCKS 1
@@ -877,6 +877,8 @@ __device__ __forceinline__ void sodecl_lanes_advance_run(real_t &t, real_t *yown
 #if SODECL_SPECULATE
     const real_t t0 = t;
     const double counter0 = counter;
+    const sodecl_i64 passes0 = passes;
+    const int capped0 = capped;
     real_t y0[SODECL_ROWS];
 #pragma unroll
     for (int k = 0; k < SODECL_ROWS; ++k) y0[k] = yown[k];
@@ -893,6 +895,8 @@ __device__ __forceinline__ void sodecl_lanes_advance_run(real_t &t, real_t *yown
         if (__ballot_sync(v.mask, finite) & v.mask) {
             real_t tc = t0;
             double cc = counter0;
+            passes = passes0;
+            capped = capped0;
 #pragma unroll
             for (int k = 0; k < SODECL_ROWS; ++k) {
                 const int r = v.lane + k * SODECL_LANES;

@@ -378,7 +378,8 @@ SystemTraits inspect_system(const std::string &src)
     t.has_vjp = defines_function(stripped, "calc_vjp");
     t.uses_listsize = std::regex_search(stripped, std::regex("\\b_listsize_\\b"));
     t.uses_division = stripped.find('/') != std::string::npos;
-    t.uses_math = std::regex_search(stripped, std::regex("\\b(native_|half_)?(sin|cos|sincos|exp)\\s*\\("));
+    t.uses_trig = std::regex_search(stripped, std::regex("\\b(native_|half_)?(sin|cos|sincos)\\s*\\("));
+    t.uses_exp = std::regex_search(stripped, std::regex("\\b(native_|half_)?exp\\s*\\("));
     return t;
 }
 
@@ -406,13 +407,15 @@ std::vector<std::string> defined_macros(const std::string &src)
 // copy of the system file that follows: copy is "spec" (the speculative copy)
 // or "full" (the plain one).  The stochastic solver takes the finer exp: beside
 // a step's noise (a logarithm, a root and a sine pair for every two processes)
-// its six instructions are few, where they cost RK4 a tenth.
+// its six instructions are few, where they cost RK4 a tenth.  The implicit
+// solvers keep the library's exp (fast_math_for).
 std::string math_macros(const std::string &copy, int solver)
 {
+    const std::string exp_name = solver == 0 ? "exp_fine" : "exp";
     std::string s;
-    for (const std::string fn : {"sin", "cos", "exp", "sincos"})
-        s += "#define " + fn + "(...) sodecl_" + copy + "_" + fn + (fn == "exp" && solver == 0 ? "_fine" : "") +
-             "(__VA_ARGS__)\n";
+    for (const std::string fn : {"sin", "cos", "sincos"})
+        s += "#define " + fn + "(...) sodecl_" + copy + "_" + fn + "(__VA_ARGS__)\n";
+    if (solver <= 2) s += "#define exp(...) sodecl_" + copy + "_" + exp_name + "(__VA_ARGS__)\n";
     return s;
 }
 
@@ -428,30 +431,48 @@ std::string undef_lines(const std::vector<std::string> &names)
 // The system file as the solvers see it: with speculative steps its
 // speculative copy first, which with the solvers' step functions lies in a
 // namespace of its own, then the plain copy.
-std::string user_text(const std::string &src, const std::string &name, const std::string &as_double, bool speculate,
+std::string user_text(const std::string &src, const std::string &name, const std::string &as_double, FastMath math,
                       int solver)
 {
     const std::string plain = (as_double.empty() ? "" : "#undef double\n");
     const std::string user = "#line 1 \"" + name + "\"\n" + src + "\n";
-    if (!speculate) return as_double + user + plain;
-    return "namespace sodecl_spec {\nSODECL_SPEC_QUOTIENT\n" + as_double + math_macros("spec", solver) + user +
-           undef_math_macros() + plain + undef_lines(defined_macros(src)) +
-           "#ifndef SODECL_STEPS_ONLY\n#define SODECL_STEPS_ONLY 1\n#define SODECL_STEPS_ONLY_HERE 1\n#endif\n"
-           "#define SODECL_SPEC_COPY 1\n#line 1 \"solvers.cuh\"\n" + kSolversSrc +
-           "\n#undef SODECL_SPEC_COPY\n#ifdef SODECL_STEPS_ONLY_HERE\n#undef SODECL_STEPS_ONLY_HERE\n"
-           "#undef SODECL_STEPS_ONLY\n#endif\n}  // namespace sodecl_spec\n" +
-           as_double + math_macros("full", solver) + user + undef_math_macros() + plain;
+    if (math == FastMath::Off) return as_double + user + plain;
+    std::string s;
+    if (math == FastMath::Speculative)
+        s = std::string("namespace sodecl_spec {\n") + (solver <= 2 ? "SODECL_SPEC_QUOTIENT\n" : "") + as_double +
+            math_macros("spec", solver) + user + undef_math_macros() + plain + undef_lines(defined_macros(src)) +
+            "#ifndef SODECL_STEPS_ONLY\n#define SODECL_STEPS_ONLY 1\n#define SODECL_STEPS_ONLY_HERE 1\n#endif\n"
+            "#define SODECL_SPEC_COPY 1\n#line 1 \"solvers.cuh\"\n" + kSolversSrc +
+            "\n#undef SODECL_SPEC_COPY\n#ifdef SODECL_STEPS_ONLY_HERE\n#undef SODECL_STEPS_ONLY_HERE\n"
+            "#undef SODECL_STEPS_ONLY\n#endif\n}  // namespace sodecl_spec\n";
+    return s + as_double + math_macros("full", solver) + user + undef_math_macros() + plain;
 }
 
-// Whether speculative steps have something to gain: a function of
-// device/fastmath.cuh or a reciprocal quotient (RK4 divides by itself) in a
-// solver whose step is a fixed sequence of evaluations.  A repeated step would
-// print twice.  One thread's arrays of more than 256 equations fill its local
-// memory already; the copy of the state would only add to it.
-bool worth_speculating(const ProgramSpec &s, const SystemTraits &t, const std::string &src)
+// What a solver can use of device/fastmath.cuh, at most `allowed`.
+//  - Euler, RK4 and Euler-Maruyama evaluate a fixed sequence: speculative steps
+//    wherever a function or a reciprocal quotient is called (RK4 divides by
+//    itself).
+//  - The implicit solvers count their passes by a test of the residual
+//    x - y - h f, which has to come out the same.  A sine of another rounding
+//    moves it by h ulp(1), far below ulp(x), so sin and cos are taken;
+//    exponentials may be large (the oculomotor burst's are), so exp and the
+//    quotient are not.  With lanes per orbit the step is a function of its own
+//    and speculates; the one-thread kernel's passes test each argument.
+//  - The adaptive solver accepts steps by an error estimate, and keeps all of
+//    the library's functions.
+// A repeated step would print twice.  One thread's arrays of more than 256
+// equations fill its local memory already; the copy of the state would only
+// add to it.
+FastMath fast_math_for(FastMath allowed, const ProgramSpec &s, bool fast_div, const SystemTraits &t,
+                       const std::string &src)
 {
-    return s.speculate && src.find("printf") == std::string::npos && (s.lanes > 1 || s.num_equat <= 256) &&
-           (t.uses_math || (s.fast_div && (t.uses_division || s.solver == 2)));
+    if (allowed == FastMath::Off || s.solver == 5 || src.find("printf") != std::string::npos) return FastMath::Off;
+    if (s.solver == 3 || s.solver == 4) {
+        if (!t.uses_trig) return FastMath::Off;
+        return s.lanes > 1 ? allowed : FastMath::Guarded;
+    }
+    const bool gain = t.uses_trig || t.uses_exp || (fast_div && (t.uses_division || s.solver == 2));
+    return gain && (s.lanes > 1 || s.num_equat <= 256) ? allowed : FastMath::Off;
 }
 
 }  // namespace
@@ -475,9 +496,9 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
     s << "#define SODECL_HAS_STOCH_ROW " << (traits.has_stoch_row ? 1 : 0) << "\n";
     s << "#define SODECL_HAS_JAC_BAND " << (traits.has_jac_band ? 1 : 0) << "\n";
     s << "#define SODECL_HAS_ROW_BAND " << (traits.has_row_band ? 1 : 0) << "\n";
-    s << "#define SODECL_SPECULATE " << (spec.speculate ? 1 : 0) << "\n";
+    s << "#define SODECL_SPECULATE " << (spec.fast_math == FastMath::Speculative ? 1 : 0) << "\n";
     s << kFastDivSrc << "\n" << kPreludeSrc << "\n" << kMathCoreSrc << "\n";
-    if (spec.speculate) s << kFastMathSrc << "\n";
+    if (spec.fast_math != FastMath::Off) s << kFastMathSrc << "\n";
     s << kThreefrySrc << "\n";
     // the reference's program defines (src/sodeclmgr.cpp:379-430); _listsize_
     // only when the system file names it, so one program serves every size
@@ -501,7 +522,7 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
     }
     const std::string as_double = spec.fast_div ? "#define double sodecl_num\n" : spec.fp32 ? "#define double float\n" : "";
     const std::string bounded = relax_parameter_bounds(system_src);
-    s << user_text(spec.fp32 ? suffix_float_literals(bounded) : bounded, "system.cl", as_double, spec.speculate,
+    s << user_text(spec.fp32 ? suffix_float_literals(bounded) : bounded, "system.cl", as_double, spec.fast_math,
                    spec.solver);
     s << "#line 1 \"solvers.cuh\"\n" << kSolversSrc << "\n";
     return s.str();
@@ -574,7 +595,8 @@ std::shared_ptr<const Program> compile_text(std::string source, bool fmad, bool 
 std::shared_ptr<const Program> compile_one(const ProgramSpec &spec, const std::string &system_src,
                                            const SystemTraits &traits)
 {
-    return compile_text(assemble(spec, system_src, traits), spec.fmad, spec.fast_div, "sodecl_orbits", spec.speculate);
+    return compile_text(assemble(spec, system_src, traits), spec.fmad, spec.fast_div, "sodecl_orbits",
+                        spec.fast_math == FastMath::Speculative);
 }
 
 }  // namespace
@@ -589,7 +611,7 @@ int batch_warp_words(const std::vector<BatchClass> &classes)
 
 namespace {
 
-std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div, bool speculate, int block_max,
+std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div, FastMath allowed, int block_max,
                            int min_blocks)
 {
     std::ostringstream s;
@@ -599,7 +621,7 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
     s << "#define SODECL_BLOCK_MAX " << block_max << "\n";
     s << "#define SODECL_BATCH_MIN_BLOCKS " << std::max(1, min_blocks) << "\n";
     s << kFastDivSrc << "\n" << kPreludeSrc << "\n" << kMathCoreSrc << "\n";
-    if (speculate) s << kFastMathSrc << "\n";
+    if (allowed != FastMath::Off) s << kFastMathSrc << "\n";
     s << kThreefrySrc << "\n" << kBatchSrc << "\n";
     static const char *per_class[] = {"SODECL_SOLVER", "SODECL_HAS_JACOBIAN", "SODECL_HAS_STOCH", "SODECL_NEWTON_MAX",
                                       "_numnoi_", "_numsteps_", "_m_dt_", "_numeq_", "_numpar_", "_epsilon1_",
@@ -610,10 +632,7 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
         const ProgramSpec &sp = classes[k].spec;
         const std::string &src = classes[k].system_src;
         const SystemTraits tr = inspect_system(src);
-        ProgramSpec gain = sp;
-        gain.fast_div = fast_div;
-        gain.speculate = speculate && sp.solver <= 2;
-        const bool spec = worth_speculating(gain, tr, src);
+        const FastMath math = fast_math_for(allowed, sp, fast_div, tr, src);
         s << "\n// ---- class " << k << "\n";
         for (const char *m : per_class) s << "#undef " << m << "\n";
         s << "#define SODECL_SOLVER " << sp.solver << "\n";
@@ -621,7 +640,7 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
         s << "#define SODECL_HAS_STOCH " << (tr.has_stoch ? 1 : 0) << "\n";
         s << "#define SODECL_NEWTON_MAX " << sp.newton_max_iter << "\n";
         s << "#define SODECL_LANES " << sp.lanes << "\n";
-        s << "#define SODECL_SPECULATE " << (spec ? 1 : 0) << "\n";
+        s << "#define SODECL_SPECULATE " << (math == FastMath::Speculative ? 1 : 0) << "\n";
         s << "#define SODECL_HAS_ROW " << (tr.has_row ? 1 : 0) << "\n";
         s << "#define SODECL_HAS_STOCH_ROW " << (tr.has_stoch_row ? 1 : 0) << "\n";
         s << "#define SODECL_HAS_JAC_BAND " << (tr.has_jac_band ? 1 : 0) << "\n";
@@ -636,7 +655,7 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
         s << l2_bound_define(sp.newton_tol, false);
         s << "namespace sodecl_cls_" << k << " {\n";
         s << user_text(relax_parameter_bounds(src), "class" + std::to_string(k) + ".cl",
-                       fast_div ? "#define double sodecl_num\n" : "", spec, sp.solver);
+                       fast_div ? "#define double sodecl_num\n" : "", math, sp.solver);
         for (const auto &m : defined_macros(src)) s << "#undef " << m << "\n";
         s << "#line 1 \"solvers.cuh\"\n" << kSolversSrc << "\n";
         s << "#define SODECL_BATCH_CLASS_BODY 1\n#line 1 \"batch.cuh\"\n" << kBatchSrc << "\n";
@@ -653,7 +672,7 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
     } else {
         s << "    double *warp_smem = nullptr;\n";
     }
-    if (speculate) s << "    sodecl_lower();\n";
+    if (allowed != FastMath::Off) s << "    sodecl_lower();\n";
     s << "    for (int k = 0; k < a.nclasses; ++k) {\n        switch (a.order[k]) {\n";
     for (size_t k = 0; k < classes.size(); ++k)
         s << "        case " << k << ": sodecl_cls_" << k << "::sodecl_class_run(a, " << k << ", warp_smem); break;\n";
@@ -728,12 +747,12 @@ std::shared_ptr<const Program> build_batch(const std::vector<BatchClass> &classe
         if (c.system_src.find("printf") != std::string::npos) fd = false;
     // as for one system: the plainer programs where a system file needs them
     for (const bool div : {true, false}) {
-        for (const bool speculate : {true, false}) {
+        for (const FastMath math : {FastMath::Speculative, FastMath::Off}) {
             if (div && !fd) continue;
-            const std::string text = assemble_batch(classes, div, speculate, block_max, min_blocks);
-            if (!div && !speculate) return compile_text(text, fmad, div, "sodecl_batch");
+            const std::string text = assemble_batch(classes, div, math, block_max, min_blocks);
+            if (!div && math == FastMath::Off) return compile_text(text, fmad, div, "sodecl_batch");
             try {
-                return compile_text(text, fmad, div, "sodecl_batch", speculate);
+                return compile_text(text, fmad, div, "sodecl_batch", math != FastMath::Off);
             } catch (const std::exception &) {
             }
         }
@@ -747,18 +766,18 @@ std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string 
     ProgramSpec s = spec;
     // the wrapper type would hand a struct to printf's varargs
     if (system_src.find("printf") != std::string::npos) s.fast_div = false;
-    s.speculate = worth_speculating(s, traits, system_src);
     // a system file that needs plain `double` (an implicit conversion, say)
     // does not compile with the wrapper, and one that declares or redefines
     // the math functions does not with fastmath.cuh's: the next plainer
     // program is built instead, the division mode kept as long as it can be
     for (const bool fast_div : {true, false}) {
-        for (const bool speculate : {true, false}) {
-            if ((fast_div && !s.fast_div) || (speculate && !s.speculate)) continue;
+        if (fast_div && !s.fast_div) continue;
+        for (const bool math : {true, false}) {
             ProgramSpec t = s;
             t.fast_div = fast_div;
-            t.speculate = speculate;
-            if (!fast_div && !speculate) return compile_one(t, system_src, traits);
+            t.fast_math = math ? fast_math_for(s.fast_math, s, fast_div, traits, system_src) : FastMath::Off;
+            if (math && t.fast_math == FastMath::Off) continue;
+            if (!fast_div && !math) return compile_one(t, system_src, traits);
             try {
                 return compile_one(t, system_src, traits);
             } catch (const std::exception &) {

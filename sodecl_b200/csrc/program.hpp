@@ -8,6 +8,14 @@
 
 namespace sodecl_b200 {
 
+// How a program evaluates its system file's sin, cos, exp and quotients
+// (device/fastmath.cuh).
+enum class FastMath {
+    Off,         // the library's functions
+    Guarded,     // device/fastmath.cuh's, each with its range test
+    Speculative  // steps on the speculative copy of the system file
+};
+
 struct ProgramSpec {
     int solver = 1;          // solver_Type numbering
     int num_equat = 0;
@@ -25,7 +33,7 @@ struct ProgramSpec {
     int block_max = 256;
     int min_blocks = 0;
     int lanes = 1;           // lanes per orbit (1, or a power of two up to 32)
-    bool speculate = false;  // steps on the speculative copy of the system file (device/fastmath.cuh)
+    FastMath fast_math = FastMath::Off;
     bool pair_stores = false;  // one thread per orbit: records two orbits per vector store
     double rtol = 1e-6;      // adaptive solver (solver 5): error tolerances and
     double atol = 1e-9;      // step attempts per record interval
@@ -54,7 +62,8 @@ struct SystemTraits {
     bool has_vjp = false;        // calc_vjp (v^T df/dy and v^T df/dp), used by the adjoint
     bool uses_listsize = false;
     bool uses_division = false;
-    bool uses_math = false;      // calls sin, cos, sincos or exp (the functions of device/fastmath.cuh)
+    bool uses_trig = false;      // calls sin, cos or sincos, and
+    bool uses_exp = false;       // exp (the functions of device/fastmath.cuh)
 };
 
 SystemTraits inspect_system(const std::string &src);

@@ -542,12 +542,8 @@ ProgramSpec make_spec(const sodecl_cfg &c)
         spec.min_blocks = std::max(1, 65536 / (spec.block_max * 85));
     spec.fast_div = reciprocal_division(c);
     spec.lanes = lanes_of(c);
-    // sin, cos and exp without branches (device/fastmath.cuh) in FP64 for the
-    // solvers whose step is a fixed sequence of evaluations.  The implicit and
-    // adaptive solvers decide by a tolerance how often they evaluate, so they
-    // keep the library's functions, and with them their pass and step counts
-    spec.speculate = !spec.fp32 && (c.solver == SODECL_EULER || c.solver == SODECL_RUNGE_KUTTA ||
-                                    c.solver == SODECL_STOCHASTIC_EULER);
+    // sin, cos, exp and quotients without branches, in FP64
+    spec.fast_math = spec.fp32 ? sodecl_b200::FastMath::Off : sodecl_b200::FastMath::Speculative;
     // paired stores need the pair's two threads at the same store with orbits
     // 2k and 2k+1: the one-thread kernel of the explicit and stochastic
     // solvers (the implicit and adaptive kernels store per lane, whenever that

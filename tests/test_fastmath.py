@@ -11,7 +11,7 @@ off."""
 import numpy as np
 import pytest
 
-from sodecl_b200 import Integrator
+from sodecl_b200 import Integrator, system_path
 
 pytestmark = pytest.mark.gpu
 
@@ -106,3 +106,14 @@ def test_runs_that_leave_the_range_are_repeated(ksteps, lanes):
         for _ in range(min(ksteps, got.shape[0] * ksteps)):
             y = y + (p[:, :1] + np.sin(y) + np.cos(y) / 2.5) * h
         done += ksteps
+
+
+@pytest.mark.parametrize("system,solver,lanes,copies", [
+    ("kuramoto", "euler", 1, 2), ("kuramoto", "rk4", 4, 2), ("kuramoto", "ie", 4, 2), ("kuramoto", "im", 8, 2),
+    ("kuramoto", "ie", 1, 1), ("oculomotor", "rk4", 1, 2), ("oculomotor", "ie", 1, 0)])
+def test_shipped_systems_compile_with_it(system, solver, lanes, copies):
+    """No compilation falls back to the plain program unnoticed."""
+    neq, npar = (8, 9) if system == "kuramoto" else (6, 6)
+    with Integrator(system_path(system), solver, dt=0.01, tspan=0.1, ksteps=5, neq=neq, npar=npar, orbits=4, lanes=lanes) as sim:
+        text = sim.program_source
+    assert text.count("#define sin(...)") == copies
