@@ -117,3 +117,22 @@ def test_shipped_systems_compile_with_it(system, solver, lanes, copies):
     with Integrator(system_path(system), solver, dt=0.01, tspan=0.1, ksteps=5, neq=neq, npar=npar, orbits=4, lanes=lanes) as sim:
         text = sim.program_source
     assert text.count("#define sin(...)") == copies
+
+
+@pytest.mark.parametrize("solver,neq,lanes", [("ie", 3, 2), ("ie", 16, 8), ("im", 5, 4), ("im", 33, 32)])
+def test_banded_solve_of_lanes_outside_its_range(solver, neq, lanes):
+    """Couplings of zero, tiny, ordinary and huge, and NaN: entries of the band
+    beyond 2^-480 and 2^480 take IEEE quotients, the others the same bits."""
+    coupling = np.array([2.0, 0.0, 1e-200, 1e160, 3.5, np.nan, 1e-150, 4.5])
+    n = coupling.size
+    rng = np.random.default_rng(neq)
+    p = np.concatenate([coupling[:, None], rng.normal(size=(n, neq))], axis=1)
+    y0 = rng.uniform(0, 2 * np.pi, (n, neq))
+    out = []
+    for many in (1, lanes):
+        with Integrator(system_path("kuramoto"), solver, dt=0.01, tspan=0.095, ksteps=2, neq=neq, npar=neq + 1,
+                        orbits=n, lanes=many, fmad=False, newton_max_iter=50) as sim:
+            sim.upload(np.zeros(n), y0, p)
+            out.append((sim.run(), *sim.status()))
+    for one, many in zip(*out):
+        np.testing.assert_array_equal(many, one)
