@@ -333,7 +333,7 @@ __device__ __forceinline__ void sodecl_step_em(real_t h, real_t t, real_t *y, re
 #endif
 
 #if SODECL_SOLVER == 5
-#if SODECL_LANES > 1 || defined(SODECL_STEPS_ONLY)
+#if SODECL_LANES > 1 || (defined(SODECL_STEPS_ONLY) && !defined(SODECL_SPEC_COPY))
 #error "the adaptive solver runs one thread per orbit, in single-system programs"
 #endif
 // Dormand-Prince 5(4) with adaptive steps (J. R. Dormand, P. J. Prince, "A
@@ -354,52 +354,32 @@ __device__ __forceinline__ void sodecl_step_em(real_t h, real_t t, real_t *y, re
 // needs more than SODECL_MAX_STEPS attempts, or a step too small to advance
 // t, fails: the state becomes NaN.
 #define SODECL_DP(c) ((real_t)(c))
-struct sodecl_dp_state {
-    real_t k1[_numeq_];  // the first stage at (t, y) (first same as last)
-    real_t t_end;        // the interval's end
-    int n;               // attempts in this interval
-    bool rejected;       // the last attempt was rejected
-};
-
-// Opens the interval of length span from t.  Returns false when it needs no
-// attempt: a diverged orbit stays as it is (t moves to the interval's end),
-// and an interval too short to advance t ends at once.
-__device__ __forceinline__ bool sodecl_dp_begin(real_t &t, const real_t *y, real_t *p, real_t &h, const real_t span,
-                                                sodecl_dp_state &st)
+// The stages of an attempted step of size hh from (t, y), with the first stage
+// k1 given: y5 <- y(t + hh), k7 <- f(t + hh, y5); returns the mean square over
+// equations of the scaled error.
+//
+// It is compiled twice where the program speculates: a lane's attempts are one
+// long chain (orbits need 40 to 6400 of them, and the longest sets the
+// launch's time), on which the compiler's divisions are branches of 200
+// cycles.  The speculative copy's quotients are straight-line code with the
+// same bits (fastmath.cuh, SODECL_EXACT_QUOTIENT); an attempt that meets a
+// number outside their range is taken again with the compiler's.
+__device__ __forceinline__ real_t sodecl_dp_quotient(real_t err, real_t sc)
 {
-    st.t_end = t + span;
-    bool finite = true;
-#pragma unroll SODECL_EQ_UNROLL
-    for (int e = 0; e < _numeq_; ++e) finite = finite && isfinite(y[e]);
-    if (!finite) {
-        t = st.t_end;
-        return false;
-    }
-    if (!(h > (real_t)0) || !isfinite(h)) h = (real_t)_m_dt_;
-    sode_system(t, const_cast<real_t *>(y), st.k1, p);
-    st.n = 0;
-    st.rejected = false;
-    return t < st.t_end;
+#ifdef SODECL_SPEC_COPY
+    bool bad = false;
+    const double q = sodecl_div_chain((double)err, (double)sc, bad);
+    sodecl_raise(bad);
+    return (real_t)q;
+#else
+    return err / sc;
+#endif
 }
 
-// One attempted step of the open interval.  Returns 0 while the interval
-// goes on, 1 when it has reached its end, 2 when it failed (state NaN, t at
-// the interval's end).
-__device__ __forceinline__ int sodecl_dp_attempt(real_t &t, real_t *y, real_t *p, real_t &h, sodecl_dp_state &st,
-                                                 sodecl_i64 &accepted)
+__device__ __forceinline__ real_t sodecl_dp_stages(real_t t, real_t *y, real_t *p, real_t hh, const real_t *k1,
+                                                   real_t *y5, real_t *k7)
 {
-    real_t k2[_numeq_], k3[_numeq_], k4[_numeq_], k5[_numeq_], k6[_numeq_], k7[_numeq_];
-    real_t yt[_numeq_], y5[_numeq_];
-    const real_t t_end = st.t_end;
-    const bool last = t + h >= t_end;
-    const real_t hh = last ? t_end - t : h;
-    if (st.n >= SODECL_MAX_STEPS || !(hh > (real_t)0) || t + hh == t) {
-#pragma unroll SODECL_EQ_UNROLL
-        for (int e = 0; e < _numeq_; ++e) y[e] = (real_t)__longlong_as_double(0x7ff8000000000000ULL);
-        t = t_end;
-        return 2;
-    }
-    real_t *k1 = st.k1;
+    real_t k2[_numeq_], k3[_numeq_], k4[_numeq_], k5[_numeq_], k6[_numeq_], yt[_numeq_];
 #pragma unroll SODECL_EQ_UNROLL
     for (int e = 0; e < _numeq_; ++e) yt[e] = y[e] + hh * (SODECL_DP(1.0 / 5.0) * k1[e]);
     sode_system(t + SODECL_DP(1.0 / 5.0) * hh, yt, k2, p);
@@ -436,10 +416,83 @@ __device__ __forceinline__ int sodecl_dp_attempt(real_t &t, real_t *y, real_t *p
                                  SODECL_DP(71.0 / 1920.0) * k4[e] + SODECL_DP(-17253.0 / 339200.0) * k5[e] +
                                  SODECL_DP(22.0 / 525.0) * k6[e] + SODECL_DP(-1.0 / 40.0) * k7[e]);
         const real_t sc = SODECL_DP(SODECL_ATOL) + SODECL_DP(SODECL_RTOL) * fmax(fabs(y[e]), fabs(y5[e]));
-        const real_t q = err / sc;
+        const real_t q = sodecl_dp_quotient(err, sc);
         acc = acc + q * q;
     }
-    const real_t err = sqrt(acc / (real_t)_numeq_);
+    return acc / (real_t)_numeq_;
+}
+
+#ifndef SODECL_SPEC_COPY
+__device__ __forceinline__ real_t sodecl_again(real_t x)
+{
+    double v = (double)x;
+    asm volatile("" : "+d"(v));
+    return (real_t)v;
+}
+
+struct sodecl_dp_state {
+    real_t k1[_numeq_];  // the first stage at (t, y) (first same as last)
+    real_t t_end;        // the interval's end
+    int n;               // attempts in this interval
+    bool rejected;       // the last attempt was rejected
+};
+
+// Opens the interval of length span from t.  Returns false when it needs no
+// attempt: a diverged orbit stays as it is (t moves to the interval's end),
+// and an interval too short to advance t ends at once.
+__device__ __forceinline__ bool sodecl_dp_begin(real_t &t, const real_t *y, real_t *p, real_t &h, const real_t span,
+                                                sodecl_dp_state &st)
+{
+    st.t_end = t + span;
+    bool finite = true;
+#pragma unroll SODECL_EQ_UNROLL
+    for (int e = 0; e < _numeq_; ++e) finite = finite && isfinite(y[e]);
+    if (!finite) {
+        t = st.t_end;
+        return false;
+    }
+    if (!(h > (real_t)0) || !isfinite(h)) h = (real_t)_m_dt_;
+    sode_system(t, const_cast<real_t *>(y), st.k1, p);
+    st.n = 0;
+    st.rejected = false;
+    return t < st.t_end;
+}
+
+// One attempted step of the open interval.  Returns 0 while the interval
+// goes on, 1 when it has reached its end, 2 when it failed (state NaN, t at
+// the interval's end).
+__device__ __forceinline__ int sodecl_dp_attempt(real_t &t, real_t *y, real_t *p, real_t &h, sodecl_dp_state &st,
+                                                 sodecl_i64 &accepted)
+{
+    real_t k7[_numeq_], y5[_numeq_];
+    const real_t t_end = st.t_end;
+    const bool last = t + h >= t_end;
+    const real_t hh = last ? t_end - t : h;
+    if (st.n >= SODECL_MAX_STEPS || !(hh > (real_t)0) || t + hh == t) {
+#pragma unroll SODECL_EQ_UNROLL
+        for (int e = 0; e < _numeq_; ++e) y[e] = (real_t)__longlong_as_double(0x7ff8000000000000ULL);
+        t = t_end;
+        return 2;
+    }
+    real_t *k1 = st.k1;
+#if SODECL_SPECULATE
+    real_t square = sodecl_spec::sodecl_dp_stages(t, y, p, hh, k1, y5, k7);
+    if (sodecl_raised()) {
+        sodecl_lower();
+        // other names for the same values: a product that both copies took
+        // from one register would not be contracted into either's additions
+        real_t y_again[_numeq_], k1_again[_numeq_];
+#pragma unroll SODECL_EQ_UNROLL
+        for (int e = 0; e < _numeq_; ++e) {
+            y_again[e] = sodecl_again(y[e]);
+            k1_again[e] = sodecl_again(k1[e]);
+        }
+        square = sodecl_dp_stages(t, y_again, p, sodecl_again(hh), k1_again, y5, k7);
+    }
+#else
+    const real_t square = sodecl_dp_stages(t, y, p, hh, k1, y5, k7);
+#endif
+    const real_t err = sqrt(square);
     real_t fac = (err > (real_t)0) ? SODECL_DP(0.9) * exp(SODECL_DP(-0.2) * log(err)) : SODECL_DP(5.0);
     fac = fmin(SODECL_DP(5.0), fmax(SODECL_DP(0.2), fac));
     if (err <= (real_t)1) {
@@ -460,6 +513,7 @@ __device__ __forceinline__ int sodecl_dp_attempt(real_t &t, real_t *y, real_t *p
     ++st.n;
     return t < t_end ? 0 : 1;
 }
+#endif  // SODECL_SPEC_COPY
 #undef SODECL_DP
 #endif
 
@@ -1159,6 +1213,9 @@ __device__ __forceinline__ bool sodecl_dp_open(const sodecl_args &a, sodecl_i64 
 extern "C" __global__ void __launch_bounds__(SODECL_BLOCK_MAX, SODECL_MIN_BLOCKS)
 sodecl_orbits(const sodecl_args a)
 {
+#if SODECL_SPECULATE
+    sodecl_lower();
+#endif
     const int lane = threadIdx.x % 32;
     const int in_warp = min(32, (int)blockDim.x - (int)(threadIdx.x / 32) * 32);
     const unsigned wmask = in_warp == 32 ? 0xffffffffu : (1u << in_warp) - 1u;

@@ -411,6 +411,7 @@ std::vector<std::string> defined_macros(const std::string &src)
 // solvers keep the library's exp (fast_math_for).
 std::string math_macros(const std::string &copy, int solver)
 {
+    if (solver == 5) return "";
     const std::string exp_name = solver == 0 ? "exp_fine" : "exp";
     std::string s;
     for (const std::string fn : {"sin", "cos", "sincos"})
@@ -439,8 +440,10 @@ std::string user_text(const std::string &src, const std::string &name, const std
     if (math == FastMath::Off) return as_double + user + plain;
     std::string s;
     if (math == FastMath::Speculative)
-        s = std::string("namespace sodecl_spec {\n") + (solver <= 2 ? "SODECL_SPEC_QUOTIENT\n" : "") + as_double +
-            math_macros("spec", solver) + user + undef_math_macros() + plain + undef_lines(defined_macros(src)) +
+        s = std::string("namespace sodecl_spec {\n") + (solver <= 2   ? "SODECL_SPEC_QUOTIENT\n"
+                                                      : solver == 5 ? "SODECL_EXACT_QUOTIENT\n"
+                                                                    : "") +
+            as_double + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_lines(defined_macros(src)) +
             "#ifndef SODECL_STEPS_ONLY\n#define SODECL_STEPS_ONLY 1\n#define SODECL_STEPS_ONLY_HERE 1\n#endif\n"
             "#define SODECL_SPEC_COPY 1\n#line 1 \"solvers.cuh\"\n" + kSolversSrc +
             "\n#undef SODECL_SPEC_COPY\n#ifdef SODECL_STEPS_ONLY_HERE\n#undef SODECL_STEPS_ONLY_HERE\n"
@@ -459,14 +462,17 @@ std::string user_text(const std::string &src, const std::string &name, const std
 //    quotient are not.  With lanes per orbit the step is a function of its own
 //    and speculates; the one-thread kernel's passes test each argument.
 //  - The adaptive solver accepts steps by an error estimate, and keeps all of
-//    the library's functions.
+//    the library's functions; its speculative copy's quotients are the IEEE
+//    quotients.  They need the wrapper, whose plain copy divides as the build
+//    says (speculative_wrapper).
 // A repeated step would print twice.  One thread's arrays of more than 256
 // equations fill its local memory already; the copy of the state would only
 // add to it.
 FastMath fast_math_for(FastMath allowed, const ProgramSpec &s, bool fast_div, const SystemTraits &t,
                        const std::string &src)
 {
-    if (allowed == FastMath::Off || s.solver == 5 || src.find("printf") != std::string::npos) return FastMath::Off;
+    if (allowed == FastMath::Off || src.find("printf") != std::string::npos) return FastMath::Off;
+    if (s.solver == 5) return s.num_equat <= 256 ? allowed : FastMath::Off;
     if (s.solver == 3 || s.solver == 4) {
         if (!t.uses_trig) return FastMath::Off;
         return s.lanes > 1 ? allowed : FastMath::Guarded;
@@ -474,6 +480,10 @@ FastMath fast_math_for(FastMath allowed, const ProgramSpec &s, bool fast_div, co
     const bool gain = t.uses_trig || t.uses_exp || (fast_div && (t.uses_division || s.solver == 2));
     return gain && (s.lanes > 1 || s.num_equat <= 256) ? allowed : FastMath::Off;
 }
+
+// Whether a program without the reciprocal quotient goes through sodecl_num all
+// the same, for its speculative copy.
+bool speculative_wrapper(const ProgramSpec &s) { return s.solver == 5 && s.fast_math == FastMath::Speculative; }
 
 }  // namespace
 
@@ -484,7 +494,9 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
     s << "#define SODECL_SOLVER " << spec.solver << "\n";
     s << "#define SODECL_FP32 " << (spec.fp32 ? 1 : 0) << "\n";
     s << "#define SODECL_RECORD_F32 " << (spec.record_f32 ? 1 : 0) << "\n";
-    s << "#define SODECL_FAST_DIV " << (spec.fast_div ? 1 : 0) << "\n";
+    const bool wrapper = spec.fast_div || speculative_wrapper(spec);
+    s << "#define SODECL_FAST_DIV " << (wrapper ? 1 : 0) << "\n";
+    s << "#define SODECL_IEEE_QUOTIENT " << (spec.fast_div ? 0 : 1) << "\n";
     s << "#define SODECL_HAS_JACOBIAN " << (traits.has_jacobian ? 1 : 0) << "\n";
     s << "#define SODECL_HAS_STOCH " << (traits.has_stoch ? 1 : 0) << "\n";
     s << "#define SODECL_NEWTON_MAX " << spec.newton_max_iter << "\n";
@@ -520,7 +532,7 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
         std::snprintf(buf, sizeof buf, "#define SODECL_RTOL %a\n#define SODECL_ATOL %a\n", spec.rtol, spec.atol);
         s << buf << "#define SODECL_MAX_STEPS " << spec.max_steps << "\n";
     }
-    const std::string as_double = spec.fast_div ? "#define double sodecl_num\n" : spec.fp32 ? "#define double float\n" : "";
+    const std::string as_double = wrapper ? "#define double sodecl_num\n" : spec.fp32 ? "#define double float\n" : "";
     const std::string bounded = relax_parameter_bounds(system_src);
     s << user_text(spec.fp32 ? suffix_float_literals(bounded) : bounded, "system.cl", as_double, spec.fast_math,
                    spec.solver);
@@ -597,6 +609,42 @@ std::shared_ptr<const Program> compile_one(const ProgramSpec &spec, const std::s
 {
     return compile_text(assemble(spec, system_src, traits), spec.fmad, spec.fast_div, "sodecl_orbits",
                         spec.fast_math == FastMath::Speculative);
+}
+
+// The sum over the program's functions of a figure of the compiler's report
+// (" bytes spill stores": registers stored to local memory).
+int reported_bytes(const Program &prog, const char *marker)
+{
+    int sum = 0;
+    for (size_t at = prog.log.find(marker); at != std::string::npos; at = prog.log.find(marker, at + 1)) {
+        size_t digits = at;
+        while (digits > 0 && prog.log[digits - 1] >= '0' && prog.log[digits - 1] <= '9') --digits;
+        sum += std::atoi(prog.log.c_str() + digits);
+    }
+    return sum;
+}
+
+// `capped`, or the program without the register cap where only that keeps
+// everything in registers.  Attempts of the adaptive solver are one long chain
+// for each lane, so their latency counts as much as occupancy: the oculomotor
+// model over 0.02 time units took 12.0 ms without the cap (228 registers)
+// against 15.1 with it at 4097 orbits, 25.2 against 32.7 at 2^17, 88 against
+// 98 at 2^20, Kuramoto of 5 phases 4.1 against 7.5 at 2^17.  Where the cap
+// spills next to nothing, or the state stays in local memory all the same (a
+// slow path of the math library keeps 40 bytes there), occupancy is worth more
+// (Kuramoto at 2^17: 3 phases 1.47 against 2.20 ms, 8 phases 17 against 22).
+std::shared_ptr<const Program> compile_uncapped(const ProgramSpec &spec, const std::string &system_src,
+                                                const SystemTraits &traits, std::shared_ptr<const Program> capped)
+{
+    if (!spec.liftable_cap || spec.fast_math != FastMath::Speculative ||
+        reported_bytes(*capped, " bytes spill stores") <= 128)
+        return capped;
+    ProgramSpec free = spec;
+    free.min_blocks = 1;
+    auto uncapped = compile_one(free, system_src, traits);
+    const bool resident = reported_bytes(*uncapped, " bytes spill stores") == 0 &&
+                          reported_bytes(*uncapped, " bytes stack frame") <= 64;
+    return resident ? uncapped : capped;
 }
 
 }  // namespace
@@ -779,7 +827,7 @@ std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string 
             if (math && t.fast_math == FastMath::Off) continue;
             if (!fast_div && !math) return compile_one(t, system_src, traits);
             try {
-                return compile_one(t, system_src, traits);
+                return compile_uncapped(t, system_src, traits, compile_one(t, system_src, traits));
             } catch (const std::exception &) {
             }
         }

@@ -525,13 +525,14 @@ ProgramSpec make_spec(const sodecl_cfg &c)
     // implicit solvers, one thread per orbit: by default at most 128 registers
     // a thread (four blocks of 128 threads on an SM); above that the Newton
     // pass's hoisted terms took more registers than the occupancy they cost
-    // The adaptive solver's kernel likewise: the oculomotor model at 2^20
-    // orbits over 0.2 time units took 199 ms at 128 registers against 212 ms
-    // uncapped (202 registers).
+    // The adaptive solver's kernel likewise, unless the cap makes its
+    // speculative attempts spill registers (program.cpp, build)
     if (spec.min_blocks == 0 && lanes_of(c) == 1 &&
         (c.solver == SODECL_IMPLICIT_EULER || c.solver == SODECL_IMPLICIT_MIDPOINT ||
-         c.solver == SODECL_DORMAND_PRINCE))
+         c.solver == SODECL_DORMAND_PRINCE)) {
         spec.min_blocks = std::max(1, 65536 / (spec.block_max * 128));
+        spec.liftable_cap = c.solver == SODECL_DORMAND_PRINCE;
+    }
     // FP64 RK4 on small systems, one thread per orbit: by default at most 85
     // registers a thread (three blocks of 256).  Measured on the oculomotor
     // model at 2^20 orbits x 10^4 steps: 397 ms against 426 ms with no cap

@@ -136,3 +136,35 @@ def test_banded_solve_of_lanes_outside_its_range(solver, neq, lanes):
             out.append((sim.run(), *sim.status()))
     for one, many in zip(*out):
         np.testing.assert_array_equal(many, one)
+
+
+@pytest.mark.parametrize("system,neq", [("kuramoto", 3), ("kuramoto", 9), ("oculomotor", 6)])
+def test_adaptive_attempts_have_the_plain_programs_bits(system, neq, tmp_path):
+    """Dividends inside, at and beyond the covered range, zero and NaN; a file
+    that mentions printf is built without speculative attempts."""
+    source = open(system_path(system)).read()
+    plain = tmp_path / "plain.cl"
+    plain.write_text(source + "\n/* printf */\n")
+    n = 45
+    rng = np.random.default_rng(neq)
+    if system == "kuramoto":
+        special = [2.0, 0.0, 5e-324, 1e-300, 2.0 ** -900, 2.0 ** 900, 1e280, np.nan, -3.0]
+        p = np.concatenate([np.resize(special, (n, 1)), rng.normal(size=(n, neq))], axis=1)
+        y0 = rng.uniform(0, 2 * np.pi, (n, neq))
+        dt = 0.01
+    else:
+        p = np.array([600.0, 9.0, 0.0045, 0.05, 110.0, 1.5]) * rng.uniform(0.5, 1.5, (n, 6))
+        p[:4, 4] = [0.0, 1e-310, 1e300, np.nan]
+        p[4:7, 5] = [1e-40, 1e40, np.inf]
+        y0 = np.tile([0.0, 0.0, 0.0, 0.0, 0.0, 5.0], (n, 1))
+        y0[::5, 5] = 1e-280
+        dt = 1e-4
+    out = []
+    for path in (system_path(system), str(plain)):
+        with Integrator(path, "dp45", dt=dt, tspan=30 * dt, ksteps=10, neq=neq, npar=p.shape[1], orbits=n,
+                        fmad=False) as sim:
+            assert ("#define SODECL_SPECULATE 1" in sim.program_source) == (path != str(plain))
+            sim.upload(np.zeros(n), y0, p)
+            out.append((sim.run(), *sim.status()))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
