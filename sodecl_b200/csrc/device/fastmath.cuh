@@ -122,9 +122,9 @@ SODECL_MATH_SINCOS_OF(sodecl_num)
 // The divisor's test is a branch of its own: it keeps the pair out of the step
 // loop, where the compiler otherwise computes it again next to its uses
 // (oculomotor RK4, 2^18 orbits x 1000 steps: 5.8 against 8.9 ms).
-__device__ __forceinline__ double sodecl_div_spec(double a, double b)
+template <class R> __device__ __forceinline__ R sodecl_div_spec(R a, R b)
 {
-    double zh, zl;
+    R zh, zl;
     sodecl_reciprocal_pair(b, zh, zl);
     if (sodecl_divisor_outside(b)) sodecl_raise(true);
     return sodecl_div_pair(a, zh, zl);

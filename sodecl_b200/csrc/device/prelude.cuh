@@ -103,7 +103,9 @@ typedef float sodecl_scalar_t;
 #else
 typedef double sodecl_scalar_t;
 #endif
-#if SODECL_FAST_DIV
+// SODECL_SPEC_NUM: sodecl_num in the speculative copy alone, whose namespace
+// declares its own real_t
+#if SODECL_FAST_DIV && !defined(SODECL_SPEC_NUM)
 typedef sodecl_num real_t;
 #else
 typedef sodecl_scalar_t real_t;

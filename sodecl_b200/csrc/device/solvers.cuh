@@ -79,7 +79,7 @@ __device__ __forceinline__ sodecl_num sodecl_qdiv(sodecl_num a, sodecl_num b) { 
 // A pivot that divides twice (the banded solve's forward multiplier and back
 // substitution): in reciprocal-division programs its reciprocal is taken once
 // and each quotient finished from it (sodecl_div_by, the IEEE quotient's bits).
-#if SODECL_FAST_DIV
+#if SODECL_FAST_DIV && !defined(SODECL_SPEC_NUM)
 __device__ __forceinline__ real_t sodecl_pivot_rcp(real_t d) { return sodecl_num((sodecl_num_t)1 / d.v); }
 __device__ __forceinline__ real_t sodecl_pdiv(real_t a, real_t d, real_t r) { return sodecl_num(sodecl_div_by(a.v, d.v, r.v)); }
 #else
@@ -553,7 +553,15 @@ __device__ __forceinline__ void sodecl_advance_run(real_t &t, real_t *y, real_t 
 #pragma unroll SODECL_EQ_UNROLL
     for (int e = 0; e < _numeq_; ++e) y0[e] = y[e];
 #pragma unroll 1
-    for (int q = 0; q < m; ++q) sodecl_spec::sodecl_advance(t, y, p, gid, counter, passes, capped);
+    for (int q = 0; q < m; ++q) {
+#ifdef SODECL_SPEC_NUM
+        // a sodecl_num is a struct of one float
+        sodecl_spec::sodecl_advance(reinterpret_cast<sodecl_num &>(t), reinterpret_cast<sodecl_num *>(y),
+                                    reinterpret_cast<sodecl_num *>(p), gid, counter, passes, capped);
+#else
+        sodecl_spec::sodecl_advance(t, y, p, gid, counter, passes, capped);
+#endif
+    }
     if (sodecl_raised()) {
         sodecl_lower();
         bool diverged = true;

@@ -481,9 +481,10 @@ std::string undef_lines(const std::vector<std::string> &names)
 // speculative copy first, which with the solvers' step functions lies in a
 // namespace of its own, then the plain copy.
 std::string user_text(const std::string &src, const std::string &name, const std::string &as_double, FastMath math,
-                      int solver)
+                      int solver, bool spec_num = false)
 {
     const std::string plain = (as_double.empty() ? "" : "#undef double\n");
+    const std::string spec_double = spec_num ? "typedef sodecl_num real_t;\n#define double sodecl_num\n" : as_double;
     const std::string user = "#line 1 \"" + name + "\"\n" + src + "\n";
     if (math == FastMath::Off) return as_double + user + plain;
     std::string s;
@@ -491,7 +492,7 @@ std::string user_text(const std::string &src, const std::string &name, const std
         s = std::string("namespace sodecl_spec {\n") + (solver <= 2   ? "SODECL_SPEC_QUOTIENT\n"
                                                       : solver == 5 ? "SODECL_EXACT_QUOTIENT\n"
                                                                     : "") +
-            as_double + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_lines(defined_macros(src)) +
+            spec_double + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_lines(defined_macros(src)) +
             "#ifndef SODECL_STEPS_ONLY\n#define SODECL_STEPS_ONLY 1\n#define SODECL_STEPS_ONLY_HERE 1\n#endif\n"
             "#define SODECL_SPEC_COPY 1\n#line 1 \"solvers.cuh\"\n" + kSolversSrc +
             "\n#undef SODECL_SPEC_COPY\n#ifdef SODECL_STEPS_ONLY_HERE\n#undef SODECL_STEPS_ONLY_HERE\n"
@@ -513,6 +514,9 @@ std::string user_text(const std::string &src, const std::string &name, const std
 //    the library's functions; its speculative copy's quotients are the IEEE
 //    quotients.  They need the wrapper, whose plain copy divides as the build
 //    says (speculative_wrapper).
+//  - FP32: the quotients of the explicit and stochastic solvers with one thread
+//    per orbit, also where the plain copy divides by IEEE division
+//    (speculative_num).  A float's functions are the library's in both copies.
 // A repeated step would print twice.  One thread's arrays of more than 256
 // equations fill its local memory already; the copy of the state would only
 // add to it.
@@ -520,18 +524,27 @@ FastMath fast_math_for(FastMath allowed, const ProgramSpec &s, bool fast_div, co
                        const std::string &src)
 {
     if (allowed == FastMath::Off || src.find("printf") != std::string::npos) return FastMath::Off;
+    if (s.fp32 && (s.solver > 2 || s.lanes > 1)) return FastMath::Off;
     if (s.solver == 5) return s.num_equat <= 256 ? allowed : FastMath::Off;
     if (s.solver == 3 || s.solver == 4) {
         if (!t.uses_trig) return FastMath::Off;
         return s.lanes > 1 ? allowed : FastMath::Guarded;
     }
-    const bool gain = t.uses_trig || t.uses_exp || (fast_div && (t.uses_division || s.solver == 2));
+    const bool quotient = t.uses_division || s.solver == 2;
+    const bool gain = s.fp32 ? quotient : t.uses_trig || t.uses_exp || (fast_div && quotient);
     return gain && (s.lanes > 1 || s.num_equat <= 256) ? allowed : FastMath::Off;
 }
 
 // Whether a program without the reciprocal quotient goes through sodecl_num all
 // the same, for its speculative copy.
 bool speculative_wrapper(const ProgramSpec &s) { return s.solver == 5 && s.fast_math == FastMath::Speculative; }
+
+// Whether the speculative copy alone goes through sodecl_num, the plain copy
+// through float.
+bool speculative_num(const ProgramSpec &s)
+{
+    return s.fp32 && !s.fast_div && s.solver <= 2 && s.fast_math == FastMath::Speculative;
+}
 
 }  // namespace
 
@@ -543,7 +556,8 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
     s << "#define SODECL_FP32 " << (spec.fp32 ? 1 : 0) << "\n";
     s << "#define SODECL_RECORD_F32 " << (spec.record_f32 ? 1 : 0) << "\n";
     const bool wrapper = spec.fast_div || speculative_wrapper(spec);
-    s << "#define SODECL_FAST_DIV " << (wrapper ? 1 : 0) << "\n";
+    s << "#define SODECL_FAST_DIV " << (wrapper || speculative_num(spec) ? 1 : 0) << "\n";
+    if (speculative_num(spec)) s << "#define SODECL_SPEC_NUM 1\n";
     s << "#define SODECL_IEEE_QUOTIENT " << (spec.fast_div ? 0 : 1) << "\n";
     s << "#define SODECL_HAS_JACOBIAN " << (traits.has_jacobian ? 1 : 0) << "\n";
     s << "#define SODECL_HAS_STOCH " << (traits.has_stoch ? 1 : 0) << "\n";
@@ -583,7 +597,7 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
     const std::string as_double = wrapper ? "#define double sodecl_num\n" : spec.fp32 ? "#define double float\n" : "";
     const std::string bounded = relax_parameter_bounds(system_src);
     s << user_text(spec.fp32 ? suffix_float_literals(bounded) : bounded, "system.cl", as_double, spec.fast_math,
-                   spec.solver);
+                   spec.solver, speculative_num(spec));
     s << "#line 1 \"solvers.cuh\"\n" << kSolversSrc << "\n";
     return s.str();
 }

@@ -550,8 +550,8 @@ ProgramSpec make_spec(const sodecl_cfg &c)
         spec.min_blocks = std::max(1, 65536 / (spec.block_max * 85));
     spec.fast_div = reciprocal_division(c);
     spec.lanes = lanes_of(c);
-    // sin, cos, exp and quotients without branches, in FP64
-    spec.fast_math = spec.fp32 ? sodecl_b200::FastMath::Off : sodecl_b200::FastMath::Speculative;
+    // sin, cos, exp and quotients without branches
+    spec.fast_math = sodecl_b200::FastMath::Speculative;
     // paired stores need the pair's two threads at the same store with orbits
     // 2k and 2k+1: the one-thread kernel of the explicit and stochastic
     // solvers (the implicit and adaptive kernels store per lane, whenever that

@@ -76,6 +76,39 @@ def test_values_at_the_edges_of_the_ranges(fmad):
     assert ulps[3][finite[3]].max() <= 1
 
 
+@pytest.mark.parametrize("division", ["ieee", "reciprocal"])
+def test_float_quotients_at_the_edges_of_the_range(division):
+    """Correctly rounded, but within 2^-19 of an ulp of the middle between two
+    floats and below 2^-100, where they may be one ulp off."""
+    a = np.array([0.0, 1e-45, 1e-40, 1.2e-38, 1e-30, 1e-8, 0.3, 1.0, 2.5, 7.0, 1e8, 1e30, 3.4e38, np.inf, np.nan], np.float32)
+    lim = np.array([2.0 ** -100, 2.0 ** 100, 2.0, 4.0], np.float32)
+    b = np.concatenate([lim, np.nextafter(lim, np.float32(0)), np.nextafter(lim, np.float32(np.inf)),
+                        (lim * (1 - 65 * 2.0 ** -24)).astype(np.float32), (lim * (1 - 64 * 2.0 ** -24)).astype(np.float32),
+                        np.array([1.0, 3.0, 6.0, 25.0, 0.0045, 1e-30, 1e30, 1e-45, 1e-38, 3.4e38, 0.0, np.inf, np.nan], np.float32)])
+    a, b = np.concatenate([a, -a]), np.concatenate([b, -b])
+    a, b = np.repeat(a, b.size), np.tile(b, a.size)
+    n = a.size
+    src = VALUES.replace("sin(p[0])", "0").replace("cos(p[0])", "0").replace("exp(p[0])", "0")
+    with Integrator(None, "euler", system_src=src, dt=1.0, tspan=0.5, ksteps=1, neq=4, npar=2, orbits=n,
+                    precision="fp32", division=division) as sim:
+        assert "#define SODECL_SPECULATE 1" in sim.program_source and sim.division == division
+        sim.upload(np.zeros(n), np.full((n, 4), -0.0), np.stack([a, b], axis=1).astype(np.float64))
+        got = sim.run()[1, 3].astype(np.float32)
+    with np.errstate(all="ignore"):
+        exact = a.astype(np.float64) / b.astype(np.float64)
+        want = a / b
+        ulp = np.spacing(np.abs(want)).astype(np.float64)
+        off = np.abs(got.astype(np.float64) - want)
+        middle = np.abs(np.abs(exact - want) / ulp - 0.5) < 2.0 ** -19
+    finite = np.isfinite(want)
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+    np.testing.assert_array_equal(got[~finite], want[~finite])
+    np.testing.assert_array_equal(np.signbit(got[~np.isnan(want)]), np.signbit(want[~np.isnan(want)]))
+    same = finite & ~middle & ((np.abs(want) >= 2.0 ** -100) | (want == 0))
+    np.testing.assert_array_equal(got[same], want[same])
+    assert np.all(off[finite] <= ulp[finite])
+
+
 @pytest.mark.parametrize("ksteps", [1, 7, 8, 9, 40])
 @pytest.mark.parametrize("lanes", [1, 4])
 def test_runs_that_leave_the_range_are_repeated(ksteps, lanes):
