@@ -1,17 +1,18 @@
 // Elementary functions as straight-line code in FP64, each on the arguments its
 // comment names.  Shared, as text, by the NVRTC programs (embedded by the
 // build; fastmath.cuh and threefry.cuh build on it) and the statically compiled
-// test kernels in aux_kernels.cu.  Self-contained: no includes.
+// test kernels in aux_kernels.cu.  Needs fastdiv.cuh before it.
 //
 // Methods: argument reduction in the manner of Cody and Waite ("Software
 // Manual for the Elementary Functions", 1980) with fused multiply-adds, and
 // minimax polynomials (Remez exchange) evaluated by Horner's rule.
-//  sin: x = n pi + r, |r| <= pi/2, sin x = (-1)^n sin r, sin r = r + r^3 P(r^2)
-//       with P of degree 7 (relative error 2^-61.6).  Reducing by pi and not
-//       by pi/2 needs two more coefficients and no choice between a sine and
-//       a cosine polynomial.  pi is held in two doubles: its tail
-//       contributes n 2^-108.
-//  cos: x = (k + 1/2) pi + r, cos x = (-1)^(k+1) sin r.
+//  sin, cos: x = n pi/2 + r, |r| <= pi/4, and of sin r = r + r^3 S(r^2) and
+//       cos r = 1 + r^2 (-1/2 + r^2 C(r^2)), S and C of degree 5 (relative errors
+//       2^-57.6 and 2^-59.6 with rounded coefficients), the one that n's parity
+//       names, with n's sign.  Both are evaluated, so that nothing branches and
+//       a sine and a cosine of one argument share the work.  pi/2 is held in
+//       three doubles, 2^-163 short of it, and |r| is at least 2^-60 for the
+//       doubles up to 2^30: r is right to its last bit next to a zero too.
 //  exp: x = n ln 2 + r, |r| <= ln 2 / 2, a polynomial of degree 11 whose first
 //       coefficients are 1, 1, 1/2 and the rounded 1/6 (relative error
 //       2^-57.2), times 2^n, added to the exponent.
@@ -20,24 +21,28 @@
 //       log (Sun Microsystems, 1993), R of degree 7 in s^2 (error 2^-59.5).
 //  sqrt: the hardware's approximate reciprocal root, one cubic step for it and
 //       the root together, and the residual's correction.
-// Against quadruple precision: sin and cos within 1.7 ulp (mean 0.33; the
-// library's within 1.44, mean 0.30), exp within 0.90 ulp (mean 0.26; the
-// library's 0.83, 0.26), log within 0.80 ulp, sqrt correctly rounded on 1.5e6
-// arguments.
+// Against quadruple precision: sin and cos within 1.47 ulp (mean 0.296; the
+// library's 1.48, 0.297 on the same arguments) up to 2^30 and next to every
+// zero, exp within 0.90 ulp (mean 0.26; the library's 0.83, 0.26), log within
+// 0.80 ulp, sqrt correctly rounded on 1.5e6 arguments.
 //
-// What bounds them is the FP64 pipe (14 instructions a sine, two cycles each
-// per warp and scheduler).  Independent sums of sines, every SM full: 8.9e11
-// sines/s against the library's 4.9e11, latency 114 cycles against 241.  The
-// coefficients sit in constant memory, which an FP64 instruction reads as an
-// operand; as literals, built in registers, those sums run at 6.6e11.
+// What bounds them is the FP64 pipe (20 instructions a sine, two cycles each
+// per warp and scheduler).  The coefficients sit in constant memory, which an
+// FP64 instruction reads as an operand.  (Reducing by pi takes 14 instructions
+// and no choice between two polynomials, but its rounding errors near pi/2 reach
+// 1.7 ulp: stochastic Kuramoto of 32 phases, 2^16 orbits x 200 steps, 18.8 ms
+// so, 24.9 ms here, 33.2 ms with the library's sine.)
 #ifndef SODECL_MATHCORE_CUH
 #define SODECL_MATHCORE_CUH
 
-__constant__ double sodecl_sin_poly[8] = {-0x1.5555555555555p-3,  0x1.11111111110c1p-7,  -0x1.a01a01a014878p-13,
-                                          0x1.71de3a5285e6ap-19,  -0x1.ae6454ca7583fp-26, 0x1.6123caeee6360p-33,
-                                          -0x1.ae430e21eac89p-41, 0x1.8827f95e04f40p-49};
-// 1/pi, 1.5 x 2^52 (adding it leaves the nearest integer in the low bits), -pi in two parts
-__constant__ double sodecl_sin_red[4] = {0x1.45f306dc9c883p-2, 0x1.8p52, -0x1.921fb54442d18p+1, -0x1.1a62633145c07p-53};
+__constant__ double sodecl_sin_poly[6] = {-0x1.5555555555548p-3,  0x1.111111110f703p-7,  -0x1.a01a019bdf0eap-13,
+                                          0x1.71de3548ea12ap-19,  -0x1.ae5e3f8b69be0p-26, 0x1.5d8749807c1ebp-33};
+__constant__ double sodecl_cos_poly[7] = {-0.5,                   0x1.555555555554bp-5,  -0x1.6c16c16c14f8ap-10,
+                                          0x1.a01a019c8390fp-16,  -0x1.27e4f7ea37964p-22, 0x1.1ee9d75291b14p-29,
+                                          -0x1.8fa465ee996e4p-37};
+// 2/pi, 1.5 x 2^52 (adding it leaves the nearest integer in the low bits), -pi/2 in three parts
+__constant__ double sodecl_sin_red[5] = {0x1.45f306dc9c883p-1, 0x1.8p52, -0x1.921fb54442d18p+0, -0x1.1a62633145c07p-54,
+                                         0x1.f1976b7ed8fbcp-110};
 __constant__ double sodecl_exp_poly[10] = {0.5,                   0x1.5555555555555p-3,  0x1.55555555536aep-5,
                                            0x1.11111111195ddp-7,  0x1.6c16c17b75711p-10, 0x1.a01a015a31628p-13,
                                            0x1.a019aee45f929p-16, 0x1.71dee995f714fp-19, 0x1.289c23e2e03a1p-22,
@@ -45,36 +50,61 @@ __constant__ double sodecl_exp_poly[10] = {0.5,                   0x1.5555555555
 // 1/ln 2, 1.5 x 2^52, -ln 2 in two parts
 __constant__ double sodecl_exp_red[4] = {0x1.71547652b82fep+0, 0x1.8p52, -0x1.62e42fefa39efp-1, -0x1.abc9e3b39803fp-56};
 
-// sin r for |r| <= pi/2 (and a little beyond), which has r's sign, a zero's
-// too; the sign bit of `flip` turns it
-__device__ __forceinline__ double sodecl_sin_poly_signed(double r, int flip)
+#ifndef SODECL_APPROXIMATIONS
+__device__ __forceinline__ double sodecl_rsqrt_approx(double x)
 {
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    return r;
+}
+#endif
+
+// x = n pi/2 + r: n's low bits, r's sign bit (and others), sin r and cos r.
+// |x| <= 2^30.
+struct sodecl_quarter {
+    int n, sign;
+    double s, c;
+};
+__device__ __forceinline__ sodecl_quarter sodecl_quarter_of(double x)
+{
+    sodecl_quarter q;
+    const double t = __fma_rn(x, sodecl_sin_red[0], sodecl_sin_red[1]);
+    const double n = __dsub_rn(t, sodecl_sin_red[1]);
+    q.n = __double2loint(t);
+    double r = __fma_rn(n, sodecl_sin_red[2], x);  // exact
+    r = __fma_rn(n, sodecl_sin_red[3], r);
+    q.sign = __double2hiint(r);  // (the last part, of the other sign, would turn -0 into 0)
+    r = __fma_rn(n, sodecl_sin_red[4], r);
     const double u = __dmul_rn(r, r);
-    double p = sodecl_sin_poly[7];
+    double s = sodecl_sin_poly[5], c = sodecl_cos_poly[6];
 #pragma unroll
-    for (int k = 6; k >= 0; --k) p = __fma_rn(p, u, sodecl_sin_poly[k]);
-    const double s = __fma_rn(__dmul_rn(r, u), p, r);
-    return __hiloint2double((__double2hiint(s) & 0x7fffffff) | ((__double2hiint(r) ^ flip) & (int)0x80000000),
-                            __double2loint(s));
+    for (int k = 4; k >= 0; --k) s = __fma_rn(s, u, sodecl_sin_poly[k]);
+#pragma unroll
+    for (int k = 5; k >= 0; --k) c = __fma_rn(c, u, sodecl_cos_poly[k]);
+    q.s = __fma_rn(__dmul_rn(r, u), s, r);
+    q.c = __fma_rn(c, u, 1.0);
+    return q;
+}
+
+// sin(r + n pi/2).  A sine has r's sign, a zero's too.
+__device__ __forceinline__ double sodecl_quarter_sin(const sodecl_quarter &q, int n)
+{
+    const double v = (n & 1) ? q.c : q.s;
+    const int sign = ((n & 1) ? 0 : q.sign) ^ (n << 30);
+    return __hiloint2double((__double2hiint(v) & 0x7fffffff) | (sign & (int)0x80000000), __double2loint(v));
 }
 
 // |x| <= 2^30
 __device__ __forceinline__ double sodecl_sin_core(double x)
 {
-    const double t = __fma_rn(x, sodecl_sin_red[0], sodecl_sin_red[1]);
-    const double n = __dsub_rn(t, sodecl_sin_red[1]);
-    double r = __fma_rn(n, sodecl_sin_red[2], x);
-    r = __fma_rn(n, sodecl_sin_red[3], r);
-    return sodecl_sin_poly_signed(r, __double2loint(t) << 31);
+    const sodecl_quarter q = sodecl_quarter_of(x);
+    return sodecl_quarter_sin(q, q.n);
 }
 
 __device__ __forceinline__ double sodecl_cos_core(double x)
 {
-    const double t = __fma_rd(x, sodecl_sin_red[0], sodecl_sin_red[1]);  // floor(x / pi)
-    const double h = __dadd_rn(__dsub_rn(t, sodecl_sin_red[1]), 0.5);
-    double r = __fma_rn(h, sodecl_sin_red[2], x);
-    r = __fma_rn(h, sodecl_sin_red[3], r);
-    return sodecl_sin_poly_signed(r, ~__double2loint(t) << 31);
+    const sodecl_quarter q = sodecl_quarter_of(x);
+    return sodecl_quarter_sin(q, q.n + 1);
 }
 
 // |x| < 708.  Fine: the reduction's and the last product's rounding errors are
@@ -113,8 +143,7 @@ __device__ __forceinline__ double sodecl_log_core(double x)
     const int k = (hi - 0x3fe6a09e) >> 20;  // 0x3fe6a09e: the high word of sqrt(1/2)
     const double f = __dsub_rn(__hiloint2double(hi - (k << 20), __double2loint(x)), 1.0);
     const double d = __dadd_rn(f, 2.0);
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    double r = sodecl_rcp_approx(d);
     const double e = __fma_rn(-d, r, 1.0);
     r = __fma_rn(r, __fma_rn(e, e, e), r);
     const double s = __dmul_rn(f, r), z = __dmul_rn(s, s);
@@ -129,8 +158,7 @@ __device__ __forceinline__ double sodecl_log_core(double x)
 // 2^-1000 < x < 2^1000
 __device__ __forceinline__ double sodecl_sqrt_core(double x)
 {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double y = sodecl_rsqrt_approx(x);
     double g = __dmul_rn(x, y), h = __dmul_rn(0.5, y);
     const double r = __fma_rn(-g, h, 0.5);
     const double c = __fma_rn(__dmul_rn(r, 1.5), r, r);
