@@ -108,7 +108,6 @@ __device__ __forceinline__ bool sodecl_exp_outside(double x)
 SODECL_MATH_FN(sin, ::sin, sodecl_trig_outside)
 SODECL_MATH_FN(cos, ::cos, sodecl_trig_outside)
 SODECL_MATH_FN(exp, ::exp, sodecl_exp_outside)
-SODECL_MATH_FN(exp_fine, ::exp, sodecl_exp_outside)
 #define SODECL_MATH_SINCOS_OF(type)                                                            \
     SODECL_MATH_SINCOS(sodecl_spec_sincos, sodecl_spec_sin, sodecl_spec_cos, type)             \
     SODECL_MATH_SINCOS(sodecl_full_sincos, sodecl_full_sin, sodecl_full_cos, type)

@@ -13,8 +13,8 @@
 //       a sine and a cosine of one argument share the work.  pi/2 is held in
 //       three doubles, 2^-163 short of it, and |r| is at least 2^-60 for the
 //       doubles up to 2^30: r is right to its last bit next to a zero too.
-//  exp: x = n ln 2 + r, |r| <= ln 2 / 2, a polynomial of degree 11 whose first
-//       coefficients are 1, 1, 1/2 and the rounded 1/6 (relative error
+//  exp: x = n ln 2 + r, |r| <= ln 2 / 2, exp r = 1 + r + r^2 P(r) with P of
+//       degree 9 (first coefficients 1/2 and the rounded 1/6, relative error
 //       2^-57.2), times 2^n, added to the exponent.
 //  log: x = m 2^k, m in [sqrt(1/2), sqrt(2)), f = m - 1, s = f / (2 + f), and
 //       log m = f - f^2/2 + s (f^2/2 + R(s^2)), the arrangement of fdlibm's
@@ -23,8 +23,8 @@
 //       the root together, and the residual's correction.
 // Against quadruple precision: sin and cos within 1.47 ulp (mean 0.296; the
 // library's 1.48, 0.297 on the same arguments) up to 2^30 and next to every
-// zero, exp within 0.90 ulp (mean 0.26; the library's 0.83, 0.26), log within
-// 0.80 ulp, sqrt correctly rounded on 1.5e6 arguments.
+// zero, exp within 0.78 ulp (mean 0.255; the library's 0.87, 0.258), log within
+// 0.87 ulp, sqrt correctly rounded on 1.5e6 arguments.
 //
 // What bounds them is the FP64 pipe (20 instructions a sine, two cycles each
 // per warp and scheduler).  The coefficients sit in constant memory, which an
@@ -107,28 +107,21 @@ __device__ __forceinline__ double sodecl_cos_core(double x)
     return sodecl_quarter_sin(q, q.n + 1);
 }
 
-// |x| < 708.  Fine: the reduction's and the last product's rounding errors are
-// kept and added (within 0.75 ulp, mean 0.255), for six more instructions.
-template <bool Fine>
-__device__ __forceinline__ double sodecl_exp_core_of(double x)
+// |x| < 708.  1 + r is taken in two parts, so that of r's and the sums'
+// rounding errors only r's own is left.
+__device__ __forceinline__ double sodecl_exp_core(double x)
 {
     const double t = __fma_rn(x, sodecl_exp_red[0], sodecl_exp_red[1]);
     const double n = __dsub_rn(t, sodecl_exp_red[1]);
-    const double r1 = __fma_rn(n, sodecl_exp_red[2], x);  // exact
-    const double r = __fma_rn(n, sodecl_exp_red[3], r1);
+    double r = __fma_rn(n, sodecl_exp_red[2], x);  // exact
+    r = __fma_rn(n, sodecl_exp_red[3], r);
     double p = sodecl_exp_poly[9];
 #pragma unroll
     for (int k = 8; k >= 0; --k) p = __fma_rn(p, r, sodecl_exp_poly[k]);
-    p = __fma_rn(p, r, 1.0);
-    double s = __fma_rn(p, r, 1.0);
-    if (Fine) {
-        const double low = __fma_rn(n, sodecl_exp_red[3], __dsub_rn(r1, r));
-        s = __dadd_rn(s, __dadd_rn(__fma_rn(p, r, __dsub_rn(1.0, s)), low));
-    }
+    const double h = __dadd_rn(1.0, r), low = __dsub_rn(r, __dsub_rn(h, 1.0));
+    const double s = __dadd_rn(h, __fma_rn(__dmul_rn(r, r), p, low));
     return __hiloint2double(__double2hiint(s) + (__double2loint(t) << 20), __double2loint(s));
 }
-__device__ __forceinline__ double sodecl_exp_core(double x) { return sodecl_exp_core_of<false>(x); }
-__device__ __forceinline__ double sodecl_exp_fine_core(double x) { return sodecl_exp_core_of<true>(x); }
 
 __constant__ double sodecl_log_poly[7] = {0x1.5555555555593p-1, 0x1.999999997fb31p-2, 0x1.2492494217a15p-2,
                                           0x1.c71c51e7f758cp-3, 0x1.7466462c93937p-3, 0x1.39a0f50122a2dp-3,

@@ -453,18 +453,15 @@ std::vector<std::string> defined_macros(const std::string &src)
 
 // The functions of device/fastmath.cuh in place of the library's, for the
 // copy of the system file that follows: copy is "spec" (the speculative copy)
-// or "full" (the plain one).  The stochastic solver takes the finer exp: beside
-// a step's noise (a logarithm, a root and a sine pair for every two processes)
-// its six instructions are few, where they cost RK4 a tenth.  The implicit
-// solvers keep the library's exp (fast_math_for).
+// or "full" (the plain one).  The implicit solvers keep the library's exp
+// (fast_math_for).
 std::string math_macros(const std::string &copy, int solver)
 {
     if (solver == 5) return "";
-    const std::string exp_name = solver == 0 ? "exp_fine" : "exp";
     std::string s;
     for (const std::string fn : {"sin", "cos", "sincos"})
         s += "#define " + fn + "(...) sodecl_" + copy + "_" + fn + "(__VA_ARGS__)\n";
-    if (solver <= 2) s += "#define exp(...) sodecl_" + copy + "_" + exp_name + "(__VA_ARGS__)\n";
+    if (solver <= 2) s += "#define exp(...) sodecl_" + copy + "_exp(__VA_ARGS__)\n";
     return s;
 }
 

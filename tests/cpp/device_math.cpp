@@ -49,4 +49,5 @@ extern "C" {
     }
 VALUES(sin)
 VALUES(cos)
+VALUES(exp)
 }
