@@ -17,14 +17,15 @@
 //       degree 9 (first coefficients 1/2 and the rounded 1/6, relative error
 //       2^-57.2), times 2^n, added to the exponent.
 //  log: x = m 2^k, m in [sqrt(1/2), sqrt(2)), f = m - 1, s = f / (2 + f), and
-//       log m = f - f^2/2 + s (f^2/2 + R(s^2)), the arrangement of fdlibm's
-//       log (Sun Microsystems, 1993), R of degree 7 in s^2 (error 2^-59.5).
+//       log m = 2 artanh s = 2 s + s^3 P(s^2), P of degree 7 (relative error
+//       2^-61.6), with the rounding errors of s and of 2 s + k ln 2 kept and
+//       added.
 //  sqrt: the hardware's approximate reciprocal root, one cubic step for it and
 //       the root together, and the residual's correction.
 // Against quadruple precision: sin and cos within 1.47 ulp (mean 0.296; the
 // library's 1.48, 0.297 on the same arguments) up to 2^30 and next to every
 // zero, exp within 0.78 ulp (mean 0.255; the library's 0.87, 0.258), log within
-// 0.87 ulp, sqrt correctly rounded on 1.5e6 arguments.
+// 0.55 ulp (the library's 0.54, both means 0.250), sqrt correctly rounded on 1.5e6 arguments.
 //
 // What bounds them is the FP64 pipe (20 instructions a sine, two cycles each
 // per warp and scheduler).  The coefficients sit in constant memory, which an
@@ -123,11 +124,11 @@ __device__ __forceinline__ double sodecl_exp_core(double x)
     return __hiloint2double(__double2hiint(s) + (__double2loint(t) << 20), __double2loint(s));
 }
 
-__constant__ double sodecl_log_poly[7] = {0x1.5555555555593p-1, 0x1.999999997fb31p-2, 0x1.2492494217a15p-2,
-                                          0x1.c71c51e7f758cp-3, 0x1.7466462c93937p-3, 0x1.39a0f50122a2dp-3,
-                                          0x1.2f0d8ea92ff11p-3};
-// ln 2 in two parts
-__constant__ double sodecl_log_red[2] = {0x1.62e42fefa39efp-1, 0x1.abc9e3b39803fp-56};
+__constant__ double sodecl_log_poly[8] = {0x1.5555555555555p-1, 0x1.9999999999dfcp-2, 0x1.249249242b70dp-2,
+                                          0x1.c71c7258cba33p-3, 0x1.745cde43ad8bap-3, 0x1.3b20a964a1f34p-3,
+                                          0x1.0f5cf550b1f53p-3, 0x1.0f61a3beb2042p-3};
+// ln 2 in two parts, the first with eleven zeros at its end: its products by k are exact
+__constant__ double sodecl_log_red[2] = {0x1.62e42fefa3800p-1, 0x1.ef35793c76730p-45};
 
 // 0 < x < infinity, x normal
 __device__ __forceinline__ double sodecl_log_core(double x)
@@ -135,17 +136,19 @@ __device__ __forceinline__ double sodecl_log_core(double x)
     const int hi = __double2hiint(x);
     const int k = (hi - 0x3fe6a09e) >> 20;  // 0x3fe6a09e: the high word of sqrt(1/2)
     const double f = __dsub_rn(__hiloint2double(hi - (k << 20), __double2loint(x)), 1.0);
-    const double d = __dadd_rn(f, 2.0);
+    const double d = __dadd_rn(f, 2.0), dlow = __dsub_rn(f, __dsub_rn(d, 2.0));
     double r = sodecl_rcp_approx(d);
     const double e = __fma_rn(-d, r, 1.0);
     r = __fma_rn(r, __fma_rn(e, e, e), r);
     const double s = __dmul_rn(f, r), z = __dmul_rn(s, s);
-    double p = sodecl_log_poly[6];
+    const double slow = __dmul_rn(__fma_rn(-s, dlow, __fma_rn(-s, d, f)), r);
+    double p = sodecl_log_poly[7];
 #pragma unroll
-    for (int q = 5; q >= 0; --q) p = __fma_rn(p, z, sodecl_log_poly[q]);
-    const double h = __dmul_rn(__dmul_rn(0.5, f), f), kd = (double)k;
-    const double t = __fma_rn(s, __fma_rn(p, z, h), __dmul_rn(kd, sodecl_log_red[1]));
-    return __fma_rn(kd, sodecl_log_red[0], __dsub_rn(f, __dsub_rn(h, t)));
+    for (int q = 6; q >= 0; --q) p = __fma_rn(p, z, sodecl_log_poly[q]);
+    const double kd = (double)k, top = __dmul_rn(kd, sodecl_log_red[0]);
+    const double v = __fma_rn(2.0, s, top), vlow = __fma_rn(2.0, s, __dsub_rn(top, v));
+    const double rest = __fma_rn(kd, sodecl_log_red[1], __fma_rn(__dmul_rn(s, z), p, __dadd_rn(slow, slow)));
+    return __dadd_rn(v, __dadd_rn(vlow, rest));
 }
 
 // 2^-1000 < x < 2^1000

@@ -50,4 +50,6 @@ extern "C" {
 VALUES(sin)
 VALUES(cos)
 VALUES(exp)
+VALUES(log)
+VALUES(sqrt)
 }
