@@ -92,7 +92,7 @@ def build(verbose=False):
     headers = [os.path.join(INCLUDE, h) for h in os.listdir(INCLUDE)] + \
               [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith((".hpp", ".inc"))] + \
               [os.path.join(CSRC, "device", h) for h in os.listdir(os.path.join(CSRC, "device"))]
-    for src in ("program.cpp", "sodecl_cuda.cpp", "batch.cpp", "sodeclmgr.cpp"):
+    for src in ("program.cpp", "speculable.cpp", "sodecl_cuda.cpp", "batch.cpp", "sodeclmgr.cpp"):
         obj = os.path.join(OBJ, src + ".o")
         cmd = ["g++"] + cxxflags + ["-c", os.path.join(CSRC, src), "-o", obj]
         d = _digest([os.path.join(CSRC, src)] + sorted(headers), " ".join(cmd))

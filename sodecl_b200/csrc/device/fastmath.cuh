@@ -9,7 +9,9 @@
 // cover, and the system file is compiled twice:
 //  - the speculative copy (namespace sodecl_spec) calls sodecl_spec_sin and
 //    so on, which compute the covered range's result and raise the thread's
-//    flag for an argument outside it (a predicated store, no branch);
+//    flag for an argument outside it (a predicated store, no branch).  What the
+//    copy computes after that is thrown away, but it runs: so only files whose
+//    loops and addresses do not hang on numbers get one (speculable.hpp);
 //  - the plain copy calls sodecl_full_sin and so on, which test the range and
 //    take the library's function outside it.
 // A run of up to SODECL_SPEC_RUN steps uses the speculative copy; a thread
@@ -49,27 +51,22 @@ __device__ __forceinline__ void sodecl_lower()
     asm volatile("st.shared.u32 [%0], %1;" ::"r"(sodecl_flag_address()), "r"(0u));
 }
 
-// The range tests read the argument's high word as a float, which is ordered
-// like it: 26.0f is the high word of 2^30, 4.19140625f that of 708.  The high
-// words of Inf, NaN and the largest numbers are a NaN or Inf then, and outside.
-__device__ __forceinline__ bool sodecl_trig_outside(double x)
-{
-    return !(fabsf(__int_as_float(__double2hiint(x))) <= 26.0f);
-}
-__device__ __forceinline__ bool sodecl_exp_outside(double x)
-{
-    return !(fabsf(__int_as_float(__double2hiint(x))) < 4.19140625f);
-}
-
-#define SODECL_MATH_FN(fn, library, outside)                                                                    \
+// Outside the covered range the speculative copy gets a value that the function
+// can have (sodecl_*_bounded), not the polynomial's: the rest of the step runs on
+// it.
+#define SODECL_MATH_FN(fn, library)                                                                             \
     __device__ __forceinline__ double sodecl_spec_##fn(double x)                                                \
     {                                                                                                           \
-        sodecl_raise(outside(x));                                                                               \
-        return sodecl_##fn##_core(x);                                                                           \
+        bool outside;                                                                                           \
+        const double v = sodecl_##fn##_bounded(x, outside);                                                     \
+        sodecl_raise(outside);                                                                                  \
+        return v;                                                                                               \
     }                                                                                                           \
     __device__ __forceinline__ double sodecl_full_##fn(double x)                                                \
     {                                                                                                           \
-        return outside(x) ? library(x) : sodecl_##fn##_core(x);                                                 \
+        bool outside;                                                                                           \
+        const double v = sodecl_##fn##_bounded(x, outside);                                                     \
+        return outside ? library(x) : v;                                                                        \
     }                                                                                                           \
     SODECL_MATH_OTHER(sodecl_spec_##fn, library)                                                                \
     SODECL_MATH_OTHER(sodecl_full_##fn, library)
@@ -105,9 +102,9 @@ __device__ __forceinline__ bool sodecl_exp_outside(double x)
         *c = cosine(x);                                                                        \
     }
 
-SODECL_MATH_FN(sin, ::sin, sodecl_trig_outside)
-SODECL_MATH_FN(cos, ::cos, sodecl_trig_outside)
-SODECL_MATH_FN(exp, ::exp, sodecl_exp_outside)
+SODECL_MATH_FN(sin, ::sin)
+SODECL_MATH_FN(cos, ::cos)
+SODECL_MATH_FN(exp, ::exp)
 #define SODECL_MATH_SINCOS_OF(type)                                                            \
     SODECL_MATH_SINCOS(sodecl_spec_sincos, sodecl_spec_sin, sodecl_spec_cos, type)             \
     SODECL_MATH_SINCOS(sodecl_full_sincos, sodecl_full_sin, sodecl_full_cos, type)

@@ -124,6 +124,43 @@ __device__ __forceinline__ double sodecl_exp_core(double x)
     return __hiloint2double(__double2hiint(s) + (__double2loint(t) << 20), __double2loint(s));
 }
 
+// The same for any argument, each result one that the function can have, and
+// whether it is the value (else `outside` is set): code that goes on with it
+// until somebody looks must not meet a negative exp or a sine beyond 1.
+// For finite |x| >= 2^30 sin and cos are next to 0.  Inf and NaN are inside.
+__device__ __forceinline__ bool sodecl_trig_outside(double x)
+{
+    const unsigned h = (unsigned)__double2hiint(x) << 1;  // 0x83a00000: 2^30, 0xffe00000: infinity
+    return h - 0x83a00000u < 0xffe00000u - 0x83a00000u;
+}
+__device__ __forceinline__ double sodecl_sin_bounded(double x, bool &outside)
+{
+    const double v = sodecl_sin_core(x);
+    outside = sodecl_trig_outside(x);
+    return __hiloint2double(outside ? 0 : __double2hiint(v), __double2loint(v));
+}
+__device__ __forceinline__ double sodecl_cos_bounded(double x, bool &outside)
+{
+    const double v = sodecl_cos_core(x);
+    outside = sodecl_trig_outside(x);
+    return __hiloint2double(outside ? 0 : __double2hiint(v), __double2loint(v));
+}
+
+// exp is 0 from -748 down and infinity from 748 up, and outside only between
+// them and 708.  The high word as a float is ordered like the number: 4.19140625f
+// is that of 708, 4.23046875f that of 748; those of the largest numbers, Inf and
+// NaN are Inf or NaN.  As an unsigned number, a NaN's exceeds infinity's.
+__device__ __forceinline__ double sodecl_exp_bounded(double x, bool &outside)
+{
+    const double v = sodecl_exp_core(x);
+    const int hi = __double2hiint(x);
+    const float m = fabsf(__int_as_float(hi));
+    const bool inside = m < 4.19140625f, negative = hi <= (int)0xfff00000;
+    outside = m >= 4.19140625f && m < 4.23046875f;
+    const int end = negative ? 0 : (int)max((unsigned)hi, 0x7ff00000u);
+    return __hiloint2double(inside ? __double2hiint(v) : end, inside ? __double2loint(v) : 0);
+}
+
 __constant__ double sodecl_log_poly[8] = {0x1.5555555555555p-1, 0x1.9999999999dfcp-2, 0x1.249249242b70dp-2,
                                           0x1.c71c7258cba33p-3, 0x1.745cde43ad8bap-3, 0x1.3b20a964a1f34p-3,
                                           0x1.0f5cf550b1f53p-3, 0x1.0f61a3beb2042p-3};

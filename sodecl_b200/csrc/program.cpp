@@ -9,6 +9,8 @@
 // by NVRTC straight to an sm_100a cubin.
 #include "program.hpp"
 
+#include "speculable.hpp"
+
 #include <nvrtc.h>
 
 #include <dlfcn.h>
@@ -403,6 +405,7 @@ SystemTraits inspect_system(const std::string &src)
     const std::string stripped = scan_code(src, [](const std::string &s) { return s; }, false);
     SystemTraits t;
     t.uses_division = stripped.find('/') != std::string::npos;
+    t.speculation_hazard = speculation_hazard(stripped);
     const std::pair<std::string_view, bool *> functions[] = {
         {"sode_system", &t.has_system},
         {"calc_jacobian", &t.has_jacobian},
@@ -514,7 +517,9 @@ std::string user_text(const std::string &src, const std::string &name, const std
 //  - FP32: the quotients of the explicit and stochastic solvers with one thread
 //    per orbit, also where the plain copy divides by IEEE division
 //    (speculative_num).  A float's functions are the library's in both copies.
-// A repeated step would print twice.  One thread's arrays of more than 256
+// A speculative copy runs on numbers that the file's functions never gave, so
+// no file whose loops or addresses hang on numbers gets one (speculable.hpp);
+// and a repeated step would print twice.  One thread's arrays of more than 256
 // equations fill its local memory already; the copy of the state would only
 // add to it.
 FastMath fast_math_for(FastMath allowed, const ProgramSpec &s, bool fast_div, const SystemTraits &t,
@@ -522,11 +527,13 @@ FastMath fast_math_for(FastMath allowed, const ProgramSpec &s, bool fast_div, co
 {
     if (allowed == FastMath::Off || src.find("printf") != std::string::npos) return FastMath::Off;
     if (s.fp32 && (s.solver > 2 || s.lanes > 1)) return FastMath::Off;
-    if (s.solver == 5) return s.num_equat <= 256 ? allowed : FastMath::Off;
+    const bool safe = t.speculation_hazard.empty();
     if (s.solver == 3 || s.solver == 4) {
         if (!t.uses_trig) return FastMath::Off;
-        return s.lanes > 1 ? allowed : FastMath::Guarded;
+        return s.lanes > 1 && safe ? allowed : FastMath::Guarded;
     }
+    if (!safe) return FastMath::Off;
+    if (s.solver == 5) return s.num_equat <= 256 ? allowed : FastMath::Off;
     const bool quotient = t.uses_division || s.solver == 2;
     const bool gain = s.fp32 ? quotient : t.uses_trig || t.uses_exp || (fast_div && quotient);
     return gain && (s.lanes > 1 || s.num_equat <= 256) ? allowed : FastMath::Off;

@@ -65,6 +65,7 @@ struct SystemTraits {
     bool uses_division = false;
     bool uses_trig = false;      // calls sin, cos or sincos, and
     bool uses_exp = false;       // exp (the functions of device/fastmath.cuh)
+    std::string speculation_hazard;  // why it gets no speculative copy (speculable.hpp), or empty
 };
 
 SystemTraits inspect_system(const std::string &src);

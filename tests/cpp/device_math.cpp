@@ -15,6 +15,7 @@
 static long long __double_as_longlong(double x) { long long b; std::memcpy(&b, &x, 8); return b; }
 static double __longlong_as_double(long long b) { double x; std::memcpy(&x, &b, 8); return x; }
 static int __float_as_int(float x) { int b; std::memcpy(&b, &x, 4); return b; }
+static unsigned max(unsigned a, unsigned b) { return a > b ? a : b; }
 static float __int_as_float(int b) { float x; std::memcpy(&x, &b, 4); return x; }
 static int __double2hiint(double x) { return (int)(__double_as_longlong(x) >> 32); }
 static int __double2loint(double x) { return (int)(__double_as_longlong(x) & 0xffffffffLL); }
@@ -52,4 +53,17 @@ VALUES(cos)
 VALUES(exp)
 VALUES(log)
 VALUES(sqrt)
+
+#define BOUNDED(fn)                                                               \
+    void fn##_bounded(const double *x, double *y, unsigned char *outside, long n) \
+    {                                                                             \
+        for (long i = 0; i < n; ++i) {                                            \
+            bool o;                                                               \
+            y[i] = sodecl_##fn##_bounded(x[i], o);                                \
+            outside[i] = o;                                                       \
+        }                                                                         \
+    }
+BOUNDED(sin)
+BOUNDED(cos)
+BOUNDED(exp)
 }
