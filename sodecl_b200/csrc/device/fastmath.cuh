@@ -133,25 +133,13 @@ template <class R> __device__ __forceinline__ R sodecl_div_spec(R a, R b)
     }                                                                                                        \
     __device__ __forceinline__ sodecl_num &operator/=(sodecl_num &a, sodecl_num b) { return a = a / b; }
 
-// The IEEE quotient's bits, for the adaptive solver's speculative copy
-// (sodecl_div_by without its branches): three instructions where the divisor
-// is loop invariant.  Covered: |b| in [2^-100, 2^100), |a| in [2^-900, 2^900)
-// or zero, where every term is a normal number.
-__device__ __forceinline__ bool sodecl_dividend_outside(double a)
-{
-    const int hi = __double2hiint(a);
-    const float m = fabsf(__int_as_float(hi));  // ordered like |a|; NaN for a NaN
-    const bool zero = ((hi & 0x7fffffff) | __double2loint(a)) == 0;
-    return !(m < __int_as_float(1923 << 20)) | ((m < __int_as_float(123 << 20)) & !zero);
-}
+// The IEEE quotient's bits, for the adaptive solver's speculative copy.
 __device__ __forceinline__ double sodecl_div_exact(double a, double b)
 {
     const double r = 1.0 / b;
-    const unsigned hb = (unsigned)__double2hiint(b) << 1;
-    if (hb - (923u << 21) >= (200u << 21)) sodecl_raise(true);
-    const double q = __dmul_rn(a, r);
-    sodecl_raise(sodecl_dividend_outside(a));
-    return __fma_rn(__fma_rn(-q, b, a), r, q);
+    if (sodecl_straight_divisor_outside(b)) sodecl_raise(true);
+    sodecl_raise(sodecl_straight_dividend_outside(a));
+    return sodecl_div_straight(a, b, r);
 }
 #define SODECL_EXACT_QUOTIENT                                                                                \
     __device__ __forceinline__ sodecl_num operator/(sodecl_num a, sodecl_num b)                              \

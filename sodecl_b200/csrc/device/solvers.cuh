@@ -686,7 +686,7 @@ __device__ __forceinline__ double sodecl_counter_plus(double counter, int c)
 // (the iterate, which the caller writes again).
 //
 // In FP64 the quotients on the two chains are branch-free (sodecl_div_chain;
-// in the back substitution Markstein's three instructions), and what they do
+// in the back substitution sodecl_div_straight), and what they do
 // not cover is noted: the group then solves again with IEEE quotients (exact),
 // whose bits they otherwise have.  A pass of 64 rows on 32 lanes (implicit Euler,
 // Kuramoto, 340 orbits): 15.5 us against 18.9 with the IEEE quotients on the
@@ -729,9 +729,8 @@ __device__ __forceinline__ bool sodecl_lanes_backward(const sodecl_lanes_view &v
         } else {
             // the pivots were tested as the forward sweep's divisors
             const double a = (double)num, r = (double)v.A[i];
-            const double q = __dmul_rn(a, r);
             bad |= sodecl_beyond_480(a) & (a != 0.0);
-            x = (real_t)__fma_rn(__fma_rn(-q, (double)v.DX[i], a), r, q);
+            x = (real_t)sodecl_signed_like(sodecl_div_straight(a, (double)v.DX[i], r), __dmul_rn(a, r));
         }
         v.B[i] = x;
     }

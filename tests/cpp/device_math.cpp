@@ -66,4 +66,20 @@ VALUES(sqrt)
 BOUNDED(sin)
 BOUNDED(cos)
 BOUNDED(exp)
+
+void chain_quotients(const double *a, const double *b, double *q, unsigned char *outside, long n)
+{
+    for (long i = 0; i < n; ++i) {
+        bool bad = false;
+        q[i] = sodecl_div_chain(a[i], b[i], bad);
+        outside[i] = bad;
+    }
+}
+void straight_quotients(const double *a, const double *b, double *q, unsigned char *outside, long n)
+{
+    for (long i = 0; i < n; ++i) {
+        q[i] = sodecl_div_straight(a[i], b[i], 1.0 / b[i]);
+        outside[i] = sodecl_straight_divisor_outside(b[i]) || sodecl_straight_dividend_outside(a[i]);
+    }
+}
 }

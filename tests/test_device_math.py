@@ -3,7 +3,7 @@ significand), on the host: random arguments over their ranges and the hard ones.
 import numpy as np
 import pytest
 
-from device_math import ulps, values
+from device_math import call, ulps, values
 
 # pi/2 in long double and the rest, for the doubles nearest to its multiples
 HALF_PI = np.longdouble("1.57079632679489661923132169163975144")
@@ -62,3 +62,56 @@ def test_log_and_sqrt_of_the_noise():
     r = -2.0 * values("log", x[x < 1])
     r = np.concatenate([r, np.exp(rng.uniform(-300, 300, 100000))])
     np.testing.assert_array_equal(values("sqrt", r), np.sqrt(r))
+
+
+def pairs(bits, count, seed):
+    """Dividends and divisors: random significands, ones near 1 and 2, quotients
+    next to the middle between two numbers (a = b m rounded, m a bit longer than a
+    number), moderate and extreme exponents, and specials in every combination."""
+    kind, word = (np.float64, np.int64) if bits == 53 else (np.float32, np.int32)
+    rng = np.random.default_rng(seed)
+    top, wide = (1 << (bits - 1)), (40 if bits == 53 else 15)
+
+    def significand():
+        m = rng.integers(top, 2 * top, count)
+        near = rng.random(count)
+        m = np.where(near < 0.1, top + rng.integers(0, 64, count), m)
+        return np.where(near > 0.9, 2 * top - 1 - rng.integers(0, 64, count), m)
+
+    a, b = significand().astype(kind), significand().astype(kind)
+    middle = (2 * significand() + 1).astype(np.longdouble) * b.astype(np.longdouble)
+    a = np.where(rng.random(count) < 0.5, a, (middle * np.ldexp(np.longdouble(1), -bits)).astype(kind))
+    a = (np.ldexp(a, rng.integers(-wide, wide, count)) * rng.choice([-1, 1], count)).astype(kind)
+    b = (np.ldexp(b, rng.integers(-wide, wide, count)) * rng.choice([-1, 1], count)).astype(kind)
+    extreme = rng.integers(0, 1 << (63 if bits == 53 else 31), count // 10).astype(word).view(kind)
+    a[:extreme.size], b[-extreme.size:] = extreme, extreme[::-1]
+    i = np.finfo(kind)
+    special = np.array([0.0, i.smallest_subnormal, i.tiny, i.max, np.inf, np.nan, 1.0, 3.0, 2.0, i.eps, 1 - i.epsneg], kind)
+    special = np.concatenate([special, -special])
+    return (np.concatenate([a, np.repeat(special, special.size)]).astype(kind),
+            np.concatenate([b, np.tile(special, special.size)]).astype(kind))
+
+
+def check_quotients(name, a, b, covered):
+    """Bit for bit, the sign of a zero too, wherever the function does not say that it is outside."""
+    q, outside = np.empty_like(a), np.empty(a.size, dtype=np.uint8)
+    call(name, a, b, q, outside)
+    with np.errstate(all="ignore"):
+        want = a / b
+    word = np.int64 if a.dtype == np.float64 else np.int32
+    inside = outside == 0
+    nan = np.isnan(want)
+    assert np.isnan(q[inside & nan]).all()
+    same = inside & ~nan
+    np.testing.assert_array_equal(q[same].view(word), want[same].view(word))
+    assert not outside[nan & (np.isnan(a) | np.isnan(b)) & covered].any()
+    assert not outside[covered & ~nan].any()
+
+
+@pytest.mark.parametrize("name", ["chain", "straight"])
+def test_quotients_have_the_ieee_quotients_bits(name):
+    a, b = pairs(53, 2000000, 4)
+    with np.errstate(all="ignore"):
+        moderate = ((np.abs(a) > 1e-20) & (np.abs(a) < 1e40) | ((a == 0) & ~np.signbit(a)) | np.isnan(a)) & \
+            (np.abs(b) > 1e-20) & (np.abs(b) < 1e28) & (np.frexp(np.abs(b))[0] != 1 - 2.0 ** -53)
+    check_quotients(name + "_quotients", a, b, moderate)
