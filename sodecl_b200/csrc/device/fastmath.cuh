@@ -115,36 +115,22 @@ SODECL_MATH_SINCOS_OF(sodecl_num)
 #endif
 
 #if SODECL_FAST_DIV
-// The divisor's test is a branch of its own: it keeps the pair out of the step
-// loop, where the compiler otherwise computes it again next to its uses
-// (oculomotor RK4, 2^18 orbits x 1000 steps: 5.8 against 8.9 ms).
+// The IEEE quotient's bits.  The divisor's test is a branch of its own: it keeps
+// the reciprocal out of the step loop, where the compiler otherwise computes it
+// again next to its uses (oculomotor RK4, 2^18 orbits x 1000 steps: 5.8 against
+// 8.9 ms).
 template <class R> __device__ __forceinline__ R sodecl_div_spec(R a, R b)
 {
-    R zh, zl;
-    sodecl_reciprocal_pair(b, zh, zl);
-    if (sodecl_divisor_outside(b)) sodecl_raise(true);
-    return sodecl_div_pair(a, zh, zl);
+    const R r = (R)1 / b;
+    if (sodecl_straight_divisor_outside(b)) sodecl_raise(true);
+    sodecl_raise(sodecl_straight_dividend_outside(a));
+    return sodecl_div_straight(a, b, r);
 }
 // the speculative copy's `/`, declared in its namespace
 #define SODECL_SPEC_QUOTIENT                                                                                 \
     __device__ __forceinline__ sodecl_num operator/(sodecl_num a, sodecl_num b)                              \
     {                                                                                                        \
         return sodecl_num(sodecl_div_spec(a.v, b.v));                                                        \
-    }                                                                                                        \
-    __device__ __forceinline__ sodecl_num &operator/=(sodecl_num &a, sodecl_num b) { return a = a / b; }
-
-// The IEEE quotient's bits, for the adaptive solver's speculative copy.
-__device__ __forceinline__ double sodecl_div_exact(double a, double b)
-{
-    const double r = 1.0 / b;
-    if (sodecl_straight_divisor_outside(b)) sodecl_raise(true);
-    sodecl_raise(sodecl_straight_dividend_outside(a));
-    return sodecl_div_straight(a, b, r);
-}
-#define SODECL_EXACT_QUOTIENT                                                                                \
-    __device__ __forceinline__ sodecl_num operator/(sodecl_num a, sodecl_num b)                              \
-    {                                                                                                        \
-        return sodecl_num(sodecl_div_exact(a.v, b.v));                                                       \
     }                                                                                                        \
     __device__ __forceinline__ sodecl_num &operator/=(sodecl_num &a, sodecl_num b) { return a = a / b; }
 #else

@@ -362,7 +362,7 @@ __device__ __forceinline__ void sodecl_step_em(real_t h, real_t t, real_t *y, re
 // long chain (orbits need 40 to 6400 of them, and the longest sets the
 // launch's time), on which the compiler's divisions are branches of 200
 // cycles.  The speculative copy's quotients are straight-line code with the
-// same bits (fastmath.cuh, SODECL_EXACT_QUOTIENT); an attempt that meets a
+// same bits (fastmath.cuh, sodecl_div_spec); an attempt that meets a
 // number outside their range is taken again with the compiler's.
 __device__ __forceinline__ real_t sodecl_dp_quotient(real_t err, real_t sc)
 {

@@ -489,9 +489,7 @@ std::string user_text(const std::string &src, const std::string &name, const std
     if (math == FastMath::Off) return as_double + user + plain;
     std::string s;
     if (math == FastMath::Speculative)
-        s = std::string("namespace sodecl_spec {\n") + (solver <= 2   ? "SODECL_SPEC_QUOTIENT\n"
-                                                      : solver == 5 ? "SODECL_EXACT_QUOTIENT\n"
-                                                                    : "") +
+        s = std::string("namespace sodecl_spec {\n") + (solver <= 2 || solver == 5 ? "SODECL_SPEC_QUOTIENT\n" : "") +
             spec_double + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_lines(defined_macros(src)) +
             "#ifndef SODECL_STEPS_ONLY\n#define SODECL_STEPS_ONLY 1\n#define SODECL_STEPS_ONLY_HERE 1\n#endif\n"
             "#define SODECL_SPEC_COPY 1\n#line 1 \"solvers.cuh\"\n" + kSolversSrc +

@@ -82,4 +82,11 @@ void straight_quotients(const double *a, const double *b, double *q, unsigned ch
         outside[i] = sodecl_straight_divisor_outside(b[i]) || sodecl_straight_dividend_outside(a[i]);
     }
 }
+void straight_quotients_f32(const float *a, const float *b, float *q, unsigned char *outside, long n)
+{
+    for (long i = 0; i < n; ++i) {
+        q[i] = sodecl_div_straight(a[i], b[i], 1.0f / b[i]);
+        outside[i] = sodecl_straight_divisor_outside(b[i]) || sodecl_straight_dividend_outside(a[i]);
+    }
+}
 }

@@ -115,3 +115,11 @@ def test_quotients_have_the_ieee_quotients_bits(name):
         moderate = ((np.abs(a) > 1e-20) & (np.abs(a) < 1e40) | ((a == 0) & ~np.signbit(a)) | np.isnan(a)) & \
             (np.abs(b) > 1e-20) & (np.abs(b) < 1e28) & (np.frexp(np.abs(b))[0] != 1 - 2.0 ** -53)
     check_quotients(name + "_quotients", a, b, moderate)
+
+
+def test_float_quotients_have_the_ieee_quotients_bits():
+    a, b = pairs(24, 2000000, 5)
+    a = np.concatenate([a, np.float32([float.fromhex("0x1.d074d8p+0")])])
+    b = np.concatenate([b, np.float32([float.fromhex("0x1.527e7cp+0")])])
+    moderate = ((np.abs(a) > 1e-20) & (np.abs(a) < 1e20) | ((a == 0) & ~np.signbit(a)) | np.isnan(a)) & (np.abs(b) > 1e-10) & (np.abs(b) < 1e10)
+    check_quotients("straight_quotients_f32", a, b, moderate)

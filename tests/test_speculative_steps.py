@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from sodecl_b200 import Integrator
+from test_device_math import pairs
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +35,29 @@ def test_quotients_keep_a_zeros_sign(solver):
     for a, b in zip(got, plain):
         np.testing.assert_array_equal(a, b)
     assert np.all(np.sign(got[0][-1].T - 1) == np.sign(want - 1))
+
+
+@pytest.mark.parametrize("lanes", [1, 2])
+@pytest.mark.parametrize("precision,division", [("fp64", "reciprocal"), ("fp64", "ieee"), ("fp32", "reciprocal"), ("fp32", "ieee")])
+def test_quotients_are_ieee_in_every_mode(precision, division, lanes):
+    """One Euler step of size 1 from -0 is the quotient itself: random pairs, pairs
+    whose quotient lies next to the middle between two numbers, and specials."""
+    a, b = pairs(53 if precision == "fp64" else 24, 200000, 6)
+    if precision == "fp32":
+        a = np.concatenate([a, np.float32([float.fromhex("0x1.d074d8p+0")])])
+        b = np.concatenate([b, np.float32([float.fromhex("0x1.527e7cp+0")])])
+    source = "double sode_system_row(int i, double t, double y[_numeq_], double p[_numpar_]) { return p[0] / p[1]; }\n" + HEAD + \
+        "\tfor (int i = 0; i < _numeq_; i++) yout[i] = sode_system_row(i, t, y, p);\n}\n"
+    n = a.size
+    with Integrator(None, "euler", system_src=source, dt=1.0, tspan=0.5, ksteps=1, neq=2, npar=2, orbits=n, lanes=lanes,
+                    precision=precision, division=division) as sim:
+        assert sim.division == division
+        sim.upload(np.zeros(n), np.full((n, 2), -0.0), np.stack([a, b], axis=1).astype(np.float64))
+        got = sim.run()[1].astype(a.dtype)
+    with np.errstate(all="ignore"):
+        want = a / b
+    word = np.int64 if precision == "fp64" else np.int32
+    nan = np.isnan(want)
+    for row in got:
+        assert np.isnan(row[nan]).all()
+        np.testing.assert_array_equal(row[~nan].view(word), want[~nan].view(word))
