@@ -413,7 +413,7 @@ __device__ __forceinline__ void sodecl_step_adjoint(double h, double t, const do
 #define SODECL_SEG_WIDTH (_numeq_ + 1)
 #endif
 
-// One step of the forward arithmetic (sodecl_advance's), recording into st
+// One step of the forward arithmetic (sodecl_advance_run's), recording into st
 // (stride n between values) unless it is null: the state and t before the
 // step and, for RK4, its three stage inputs.  The forward sweep and the
 // segment recomputation both step through here, so they agree bit for bit.
@@ -440,7 +440,7 @@ __device__ __forceinline__ void sodecl_adjoint_step(real_t &t, real_t *y, real_t
             st[(3 * _numeq_ + 1 + e) * n] = (double)x4[e];
         }
 #else
-    sodecl_advance(t, y, p, i, counter, passes, capped);
+    sodecl_advance_run(t, y, p, i, counter, passes, capped, 1);
 #endif
 }
 

@@ -242,15 +242,7 @@ __device__ __forceinline__ void sodecl_class_run(const sodecl_batch_args &a, con
         const sodecl_i64 gid = a.orbit_id ? a.orbit_id[item] : item;
         sodecl_i64 passes = 0;
         int capped = 0;
-#if SODECL_SPECULATE
-#pragma unroll 1
-        for (long long s = 0; s < left; s += SODECL_SPEC_RUN)
-            sodecl_lanes_advance_run(t, yown, v, gid, counter, passes, capped,
-                                     (int)min(left - s, (long long)SODECL_SPEC_RUN));
-#else
-#pragma unroll 1
-        for (long long s = 0; s < left; ++s) sodecl_lanes_advance(t, yown, v, gid, counter, passes, capped);
-#endif
+        sodecl_lanes_advance_run(t, yown, v, gid, counter, passes, capped, left);
         int nonfinite = 0;
 #pragma unroll
         for (int q = 0; q < SODECL_ROWS; ++q) {

@@ -1,6 +1,6 @@
 // sin, cos, exp and the quotient for the system files of the explicit and
-// stochastic solvers, sin and cos for those of the implicit solvers, without
-// branches.
+// stochastic solvers, sin and cos for those of the implicit solvers, the
+// quotient for those of the adaptive solver, without branches.
 //
 // The math library's functions end in a branch to a slow path for rare
 // arguments, and so does the reciprocal quotient, so the compiler cannot
@@ -12,15 +12,18 @@
 //    flag for an argument outside it (a predicated store, no branch).  What the
 //    copy computes after that is thrown away, but it runs: so only files whose
 //    loops and addresses do not hang on numbers get one (speculable.hpp);
-//  - the plain copy calls sodecl_full_sin and so on, which test the range and
-//    take the library's function outside it.
-// A run of up to SODECL_SPEC_RUN steps uses the speculative copy; a thread
-// whose flag is up afterwards repeats the run with the plain copy from the
-// same state (solvers.cuh).  Covered arguments give the same value in both
-// copies, so the result depends on the orbit's own state alone.  An orbit that
-// has diverged, every component NaN, stays so whatever its right-hand side
-// returns (y + ... is NaN), so its flag is ignored.  Programs without
-// speculative steps (the one-thread implicit kernel) use the plain copy alone.
+//  - the plain copy calls sodecl_plain_sin and so on, which test the range, and
+//    outside it take the library's function and raise the flag too.
+// A step whose speculative copy raised the flag counts as the plain copy takes
+// it, from the same state (solvers.cuh).  Covered arguments give the same function
+// values in both copies, but the compiler may contract the products around them
+// differently; since the step's own state decides which copy counts, results do
+// not depend on where a run, a launch or a record interval began.  After a plain
+// step the next one is tried with the plain copy first; it counts if it raises
+// the flag too, else the speculative copy decides again.  So an orbit that stays
+// outside pays for the plain copy alone.
+// Programs without speculative steps (the one-thread implicit kernel) call
+// sodecl_full_sin and so on, the plain copy's values without the flag.
 #ifndef SODECL_FASTMATH_CUH
 #define SODECL_FASTMATH_CUH
 
@@ -39,6 +42,21 @@ __device__ __forceinline__ void sodecl_raise(bool outside)
 {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared.u32 [%1], %0;\n\t}"
                  ::"r"((unsigned)outside), "r"(sodecl_flag_address()));
+}
+// sodecl_straight_dividend_outside and the raise
+__device__ __forceinline__ void sodecl_raise_dividend(double a)
+{
+    const unsigned hi = (unsigned)__double2hiint(a);
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\tsetp.ge.and.u32 p, %1, 0xe1000000, p;\n\t"
+                 "@p st.shared.u32 [%2], %0;\n\t}"
+                 ::"r"(hi | (unsigned)__double2loint(a)), "r"((hi << 1) - (123u << 21)), "r"(sodecl_flag_address()));
+}
+__device__ __forceinline__ void sodecl_raise_dividend(float a)
+{
+    const unsigned bits = (unsigned)__float_as_int(a);
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\tsetp.ge.and.u32 p, %1, 0xcc000000, p;\n\t"
+                 "@p st.shared.u32 [%2], %0;\n\t}"
+                 ::"r"(bits), "r"((bits << 1) - (25u << 24)), "r"(sodecl_flag_address()));
 }
 __device__ __forceinline__ bool sodecl_raised()
 {
@@ -62,6 +80,13 @@ __device__ __forceinline__ void sodecl_lower()
         sodecl_raise(outside);                                                                                  \
         return v;                                                                                               \
     }                                                                                                           \
+    __device__ __forceinline__ double sodecl_plain_##fn(double x)                                               \
+    {                                                                                                           \
+        bool outside;                                                                                           \
+        const double v = sodecl_##fn##_bounded(x, outside);                                                     \
+        if (outside) sodecl_raise(true);                                                                        \
+        return outside ? library(x) : v;                                                                        \
+    }                                                                                                           \
     __device__ __forceinline__ double sodecl_full_##fn(double x)                                                \
     {                                                                                                           \
         bool outside;                                                                                           \
@@ -69,6 +94,7 @@ __device__ __forceinline__ void sodecl_lower()
         return outside ? library(x) : v;                                                                        \
     }                                                                                                           \
     SODECL_MATH_OTHER(sodecl_spec_##fn, library)                                                                \
+    SODECL_MATH_OTHER(sodecl_plain_##fn, library)                                                               \
     SODECL_MATH_OTHER(sodecl_full_##fn, library)
 // the other argument types as the library's own overloads take them: float
 // stays float, integers go through double
@@ -107,6 +133,7 @@ SODECL_MATH_FN(cos, ::cos)
 SODECL_MATH_FN(exp, ::exp)
 #define SODECL_MATH_SINCOS_OF(type)                                                            \
     SODECL_MATH_SINCOS(sodecl_spec_sincos, sodecl_spec_sin, sodecl_spec_cos, type)             \
+    SODECL_MATH_SINCOS(sodecl_plain_sincos, sodecl_plain_sin, sodecl_plain_cos, type)          \
     SODECL_MATH_SINCOS(sodecl_full_sincos, sodecl_full_sin, sodecl_full_cos, type)
 SODECL_MATH_SINCOS_OF(double)
 SODECL_MATH_SINCOS_OF(float)
@@ -123,18 +150,40 @@ template <class R> __device__ __forceinline__ R sodecl_div_spec(R a, R b)
 {
     const R r = (R)1 / b;
     if (sodecl_straight_divisor_outside(b)) sodecl_raise(true);
-    sodecl_raise(sodecl_straight_dividend_outside(a));
+    sodecl_raise_dividend(a);
     return sodecl_div_straight(a, b, r);
 }
-// the speculative copy's `/`, declared in its namespace
-#define SODECL_SPEC_QUOTIENT                                                                                 \
+template <class R> __device__ __forceinline__ R sodecl_div_spec_literal(R a, R b)
+{
+    const R r = (R)1 / b;
+    if (sodecl_straight_divisor_outside(b) || sodecl_straight_dividend_outside(a)) sodecl_raise(true);
+    return sodecl_div_straight(a, b, r);
+}
+template <class R> __device__ __forceinline__ R sodecl_div_plain(R a, R b)
+{
+    const R r = (R)1 / b;
+    if (!sodecl_straight_divisor_outside(b) && !sodecl_straight_dividend_outside(a)) return sodecl_div_straight(a, b, r);
+    sodecl_raise(true);
+    return a / b;
+}
+// each copy's `/`, declared where the copy stands
+#define SODECL_COPY_QUOTIENT(divide)                                                                         \
     __device__ __forceinline__ sodecl_num operator/(sodecl_num a, sodecl_num b)                              \
     {                                                                                                        \
-        return sodecl_num(sodecl_div_spec(a.v, b.v));                                                        \
+        return sodecl_num(divide(a.v, b.v));                                                                 \
     }                                                                                                        \
     __device__ __forceinline__ sodecl_num &operator/=(sodecl_num &a, sodecl_num b) { return a = a / b; }
+// (a dividend of a scalar type is a literal, whose test the compiler takes)
+#define SODECL_SPEC_QUOTIENT                                                                                 \
+    SODECL_COPY_QUOTIENT(sodecl_div_spec)                                                                    \
+    template <class A> __device__ __forceinline__ sodecl_num operator/(A a, sodecl_num b)                    \
+    {                                                                                                        \
+        return sodecl_num(sodecl_div_spec_literal((sodecl_num_t)a, b.v));                                    \
+    }
+#define SODECL_PLAIN_QUOTIENT SODECL_COPY_QUOTIENT(sodecl_div_plain)
 #else
 #define SODECL_SPEC_QUOTIENT
+#define SODECL_PLAIN_QUOTIENT
 #endif
 
 #endif

@@ -67,12 +67,10 @@ __device__ __forceinline__ bool operator==(sodecl_num a, sodecl_num b) { return 
 __device__ __forceinline__ bool operator!=(sodecl_num a, sodecl_num b) { return a.v != b.v; }
 }  // namespace sodecl_numeric
 using sodecl_numeric::sodecl_num;
-#if SODECL_IEEE_QUOTIENT
-__device__ __forceinline__ sodecl_num operator/(sodecl_num a, sodecl_num b) { return sodecl_num(a.v / b.v); }
-#else
+#if !SODECL_COPY_QUOTIENTS  // (else each copy of the system file brings its own)
 __device__ __forceinline__ sodecl_num operator/(sodecl_num a, sodecl_num b) { return sodecl_num(sodecl_div_rcp(a.v, b.v)); }
-#endif
 __device__ __forceinline__ sodecl_num &operator/=(sodecl_num &a, sodecl_num b) { return a = a / b; }
+#endif
 #define SODECL_NUM_UNARY(fn) \
     __device__ __forceinline__ sodecl_num fn(sodecl_num a) { return sodecl_num(::fn(a.v)); }
 SODECL_NUM_UNARY(exp) SODECL_NUM_UNARY(exp2) SODECL_NUM_UNARY(expm1) SODECL_NUM_UNARY(log)

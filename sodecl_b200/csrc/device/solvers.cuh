@@ -51,13 +51,6 @@ template <> struct sodecl_pair_of<float> { typedef float2 type; };
 #ifndef SODECL_SPECULATE
 #define SODECL_SPECULATE 0
 #endif
-// Steps between two looks at a thread's flag.  A look costs a shared-memory
-// load and a branch on the step's chain, and a copy of the state before it; a
-// flag repeats the whole run.  (Oculomotor RK4 where nearly every orbit
-// diverges, 2^18 orbits x 1000 steps of dt 1e-3: 7.6 ms with 8, 8.0 with 16,
-// 11.8 with 64; at a stable step the three are within 1 %.)
-#undef SODECL_SPEC_RUN
-#define SODECL_SPEC_RUN 8
 #if SODECL_PAIR_STORES && (SODECL_LANES != 1 || SODECL_SOLVER > 2)
 #error "paired record stores serve the one-thread kernel of the explicit and stochastic solvers"
 #endif
@@ -362,13 +355,16 @@ __device__ __forceinline__ void sodecl_step_em(real_t h, real_t t, real_t *y, re
 // long chain (orbits need 40 to 6400 of them, and the longest sets the
 // launch's time), on which the compiler's divisions are branches of 200
 // cycles.  The speculative copy's quotients are straight-line code with the
-// same bits (fastmath.cuh, sodecl_div_spec); an attempt that meets a
-// number outside their range is taken again with the compiler's.
+// same bits (fastmath.cuh, sodecl_div_spec); an attempt that meets a number
+// outside their range is taken again with the plain copy.
 __device__ __forceinline__ real_t sodecl_dp_quotient(real_t err, real_t sc)
 {
-#ifdef SODECL_SPEC_COPY
+#if SODECL_SPECULATE
     bool bad = false;
-    const double q = sodecl_div_chain((double)err, (double)sc, bad);
+    double q = sodecl_div_chain((double)err, (double)sc, bad);
+#ifndef SODECL_SPEC_COPY
+    if (bad) q = (double)err / (double)sc;
+#endif
     sodecl_raise(bad);
     return (real_t)q;
 #else
@@ -423,18 +419,13 @@ __device__ __forceinline__ real_t sodecl_dp_stages(real_t t, real_t *y, real_t *
 }
 
 #ifndef SODECL_SPEC_COPY
-__device__ __forceinline__ real_t sodecl_again(real_t x)
-{
-    double v = (double)x;
-    asm volatile("" : "+d"(v));
-    return (real_t)v;
-}
-
 struct sodecl_dp_state {
     real_t k1[_numeq_];  // the first stage at (t, y) (first same as last)
     real_t t_end;        // the interval's end
     int n;               // attempts in this interval
     bool rejected;       // the last attempt was rejected
+    bool plain;          // take the next attempt with the plain copy (fastmath.cuh)
+    bool tried;          // and it has been taken with the other
 };
 
 // Opens the interval of length span from t.  Returns false when it needs no
@@ -453,13 +444,16 @@ __device__ __forceinline__ bool sodecl_dp_begin(real_t &t, const real_t *y, real
     }
     if (!(h > (real_t)0) || !isfinite(h)) h = (real_t)_m_dt_;
     sode_system(t, const_cast<real_t *>(y), st.k1, p);
+#if SODECL_SPECULATE
+    sodecl_lower();  // the plain copy's flag: no choice to make here
+#endif
     st.n = 0;
     st.rejected = false;
     return t < st.t_end;
 }
 
-// One attempted step of the open interval.  Returns 0 while the interval
-// goes on, 1 when it has reached its end, 2 when it failed (state NaN, t at
+// One attempted step of the open interval (or none yet, in a speculative
+// program whose other copy has to decide).  Returns 0 while the interval goes on, 1 when it has reached its end, 2 when it failed (state NaN, t at
 // the interval's end).
 __device__ __forceinline__ int sodecl_dp_attempt(real_t &t, real_t *y, real_t *p, real_t &h, sodecl_dp_state &st,
                                                  sodecl_i64 &accepted)
@@ -476,19 +470,17 @@ __device__ __forceinline__ int sodecl_dp_attempt(real_t &t, real_t *y, real_t *p
     }
     real_t *k1 = st.k1;
 #if SODECL_SPECULATE
-    real_t square = sodecl_spec::sodecl_dp_stages(t, y, p, hh, k1, y5, k7);
-    if (sodecl_raised()) {
-        sodecl_lower();
-        // other names for the same values: a product that both copies took
-        // from one register would not be contracted into either's additions
-        real_t y_again[_numeq_], k1_again[_numeq_];
-#pragma unroll SODECL_EQ_UNROLL
-        for (int e = 0; e < _numeq_; ++e) {
-            y_again[e] = sodecl_again(y[e]);
-            k1_again[e] = sodecl_again(k1[e]);
-        }
-        square = sodecl_dp_stages(t, y_again, p, sodecl_again(hh), k1_again, y5, k7);
+    // an attempt whose copy does not count is none: the next call takes the other
+    real_t square;
+    if (st.plain) square = sodecl_dp_stages(t, y, p, hh, k1, y5, k7);
+    else square = sodecl_spec::sodecl_dp_stages(t, y, p, hh, k1, y5, k7);
+    const bool up = sodecl_raised();
+    if (up) sodecl_lower();
+    if (st.plain ? !up && !st.tried : up) {
+        st.plain = st.tried = !st.plain;
+        return 0;
     }
+    st.tried = false;
 #else
     const real_t square = sodecl_dp_stages(t, y, p, hh, k1, y5, k7);
 #endif
@@ -517,13 +509,10 @@ __device__ __forceinline__ int sodecl_dp_attempt(real_t &t, real_t *y, real_t *p
 #undef SODECL_DP
 #endif
 
-// One step of the configured solver from (t, y): y <- y(t + h), t <- t + h,
-// with t advanced as the reference's callers advance it
-// (solver_caller.cl:38, stochastic_solver_caller.cl:71).
-__device__ __forceinline__ void sodecl_advance(real_t &t, real_t *y, real_t *p, sodecl_i64 gid, double &counter,
-                                               sodecl_i64 &passes, int &capped)
+// The state one step of the configured solver after (t, y).
+__device__ __forceinline__ void sodecl_new_state(real_t t, real_t *y, real_t *p, sodecl_i64 gid, double &counter,
+                                                 sodecl_i64 &passes, int &capped, real_t *ynew)
 {
-    real_t ynew[_numeq_];
 #if SODECL_SOLVER == 1
     sodecl_step_euler(_m_dt_, t, y, ynew, p);
 #elif SODECL_SOLVER == 2
@@ -535,53 +524,144 @@ __device__ __forceinline__ void sodecl_advance(real_t &t, real_t *y, real_t *p, 
     sodecl_draw_noise(gid, counter, sqrt((real_t)_m_dt_), noise);
     sodecl_step_em(_m_dt_, t, y, ynew, p, noise);
 #endif
+}
+
+#ifndef SODECL_SPEC_COPY
+__device__ __forceinline__ void sodecl_take(real_t &t, real_t *y, const real_t *ynew)
+{
     t = t + _m_dt_;
 #pragma unroll SODECL_EQ_UNROLL
     for (int e = 0; e < _numeq_; ++e) y[e] = ynew[e];
 }
 
-#ifndef SODECL_SPEC_COPY
-// m steps of the configured solver (m at most SODECL_SPEC_RUN in speculative
-// programs).
+#if SODECL_SPECULATE && SODECL_LANES == 1
+// A step on the speculative copy (a sodecl_num is a struct of one scalar).
+__device__ __forceinline__ void sodecl_spec_state(real_t t, real_t *y, real_t *p, sodecl_i64 gid, double &counter,
+                                                  sodecl_i64 &passes, int &capped, real_t *ynew)
+{
+#ifdef SODECL_SPEC_NUM
+    sodecl_spec::sodecl_new_state(reinterpret_cast<sodecl_num &>(t), reinterpret_cast<sodecl_num *>(y),
+                                  reinterpret_cast<sodecl_num *>(p), gid, counter, passes, capped,
+                                  reinterpret_cast<sodecl_num *>(ynew));
+#else
+    sodecl_spec::sodecl_new_state(t, y, p, gid, counter, passes, capped, ynew);
+#endif
+}
+
+// The same value under another name.
+__device__ __forceinline__ double sodecl_again(double x)
+{
+    asm volatile("" : "+d"(x));
+    return x;
+}
+__device__ __forceinline__ float sodecl_again(float x)
+{
+    asm volatile("" : "+f"(x));
+    return x;
+}
+#if SODECL_FAST_DIV
+__device__ __forceinline__ sodecl_num sodecl_again(sodecl_num x) { return sodecl_num(sodecl_again(x.v)); }
+#endif
+
+// Every component NaN: y + ... is NaN whatever the right-hand side gives.
+__device__ __forceinline__ bool sodecl_diverged(const real_t *y)
+{
+    bool all = true;
+#pragma unroll SODECL_EQ_UNROLL
+    for (int e = 0; e < _numeq_; ++e) all = all && y[e] != y[e];
+    return all;
+}
+
+#endif
+
+// m steps: y <- y(t + m h), with t advanced as the reference's callers advance
+// it (solver_caller.cl:38, stochastic_solver_caller.cl:71).
+//
+// Speculative programs run some steps on the speculative copy before they look
+// at the flag; where it is up, they take the same steps again one by one, and the
+// one that raises it with the plain copy.  (A look after every step keeps two
+// states through the step's end and both copies in one loop: oculomotor RK4, 2^20
+// orbits x 1000 steps, 33 ms against 28.7.)  A look costs Euler 1 % every eight
+// steps, and RK4 as much every four; where nearly every orbit diverges, each in a
+// step of its own, RK4's take 34.6 ms with 4 and 36.7 with 8 (dt 1e-3).  RK4's
+// stages fill the registers in FP64, so the run's first state waits in local memory
+// there; Euler's do not, and that store costs it as much as a step.
+#undef SODECL_SPEC_RUN
+#if SODECL_SOLVER == 2 && !SODECL_FP32
+#define SODECL_SPEC_RUN 4
+#else
+#define SODECL_SPEC_RUN 8
+#endif
 __device__ __forceinline__ void sodecl_advance_run(real_t &t, real_t *y, real_t *p, sodecl_i64 gid, double &counter,
                                                    sodecl_i64 &passes, int &capped, int m)
 {
+    real_t ynew[_numeq_];
 #if SODECL_SPECULATE && SODECL_LANES == 1
-    const real_t t0 = t;
-    const double counter0 = counter;
-    real_t y0[_numeq_];
-#pragma unroll SODECL_EQ_UNROLL
-    for (int e = 0; e < _numeq_; ++e) y0[e] = y[e];
+    int left = m;    // steps to take
+    int singly = 0;  // of them, so many one by one
 #pragma unroll 1
-    for (int q = 0; q < m; ++q) {
-#ifdef SODECL_SPEC_NUM
-        // a sodecl_num is a struct of one float
-        sodecl_spec::sodecl_advance(reinterpret_cast<sodecl_num &>(t), reinterpret_cast<sodecl_num *>(y),
-                                    reinterpret_cast<sodecl_num *>(p), gid, counter, passes, capped);
-#else
-        sodecl_spec::sodecl_advance(t, y, p, gid, counter, passes, capped);
+    while (left > 0) {
+        struct { real_t t, y[_numeq_]; double counter; } start;
+        start.t = t;
+        start.counter = counter;
+#pragma unroll SODECL_EQ_UNROLL
+        for (int e = 0; e < _numeq_; ++e) start.y[e] = y[e];
+#if SODECL_SOLVER == 2 && !SODECL_FP32
+        asm volatile("" ::"l"(&start) : "memory");  // not in registers
 #endif
-    }
-    if (sodecl_raised()) {
-        sodecl_lower();
-        bool diverged = true;
-#pragma unroll SODECL_EQ_UNROLL
-        for (int e = 0; e < _numeq_; ++e) diverged = diverged && y0[e] != y0[e];
-        if (!diverged) {
-            // (as a function of its own this cost the step loop more registers
-            // and spills: oculomotor RK4, 2^18 orbits x 1000 steps, 5.72
-            // against 5.67 ms, and 7.5 against 6.6 ms at dt 1e-3)
-            real_t tc = t0;
-            double cc = counter0;
-#pragma unroll SODECL_EQ_UNROLL
-            for (int e = 0; e < _numeq_; ++e) y[e] = y0[e];
 #pragma unroll 1
-            for (int q = 0; q < m; ++q) sodecl_advance(tc, y, p, gid, cc, passes, capped);
+        for (int k = singly > 0 ? 1 : min(left, SODECL_SPEC_RUN); k > 0; --k) {
+            sodecl_spec_state(t, y, p, gid, counter, passes, capped, ynew);
+            sodecl_take(t, y, ynew);
+        }
+        const int run = singly > 0 ? 1 : min(left, SODECL_SPEC_RUN);
+        if (!sodecl_raised()) {
+            left -= run;
+            singly = max(singly - 1, 0);
+            continue;
+        }
+        sodecl_lower();
+        if (sodecl_diverged(start.y)) {
+            left -= run;
+            singly = max(singly - 1, 0);
+            continue;
+        }
+        t = start.t;
+        counter = start.counter;
+#pragma unroll SODECL_EQ_UNROLL
+        for (int e = 0; e < _numeq_; ++e) y[e] = start.y[e];
+        if (run > 1) {
+            singly = run;
+            continue;
+        }
+        // this step by the plain copy, and the next ones for as long as it
+        // raises the flag too
+        singly = 0;
+        bool first = true;
+#pragma unroll 1
+        while (left > 0) {
+            // (where a launch takes single steps, the compiler would share products of
+            // the state between the two copies, and contract neither)
+            double c = counter;
+            t = sodecl_again(t);
+#pragma unroll SODECL_EQ_UNROLL
+            for (int e = 0; e < _numeq_; ++e) y[e] = sodecl_again(y[e]);
+            sodecl_new_state(t, y, p, gid, c, passes, capped, ynew);
+            const bool up = sodecl_raised();
+            sodecl_lower();
+            if (!first && (!up || sodecl_diverged(y))) break;
+            first = false;
+            counter = c;
+            sodecl_take(t, y, ynew);
+            --left;
         }
     }
 #else
 #pragma unroll 1
-    for (int q = 0; q < m; ++q) sodecl_advance(t, y, p, gid, counter, passes, capped);
+    for (int q = 0; q < m; ++q) {
+        sodecl_new_state(t, y, p, gid, counter, passes, capped, ynew);
+        sodecl_take(t, y, ynew);
+    }
 #endif
 }
 #endif  // SODECL_SPEC_COPY
@@ -815,6 +895,10 @@ __device__ __forceinline__ int sodecl_lanes_newton(real_t h, real_t t, const rea
             if (row < _numeq_) r[k] = x[k] - yown[k] - sode_system_row(row, t, at, v.P) * h;
         }
 #endif
+#ifdef SODECL_SPEC_COPY
+        // a pass on numbers that do not count: no more of them
+        if (__ballot_sync(v.mask, sodecl_raised()) & v.mask) break;
+#endif
         // the residual norm in row order, every lane of the group the same
         real_t norm = 0;
 #pragma unroll
@@ -870,13 +954,13 @@ __device__ __forceinline__ int sodecl_lanes_newton(real_t h, real_t t, const rea
 }
 #endif
 
-// One step of the configured solver for the group's orbit: every lane of the
-// group (all of v.mask) calls it together.
-__device__ __forceinline__ void sodecl_lanes_advance(real_t &t, real_t *yown, const sodecl_lanes_view &v, sodecl_i64 gid,
-                                                     double &counter, sodecl_i64 &passes, int &capped)
+// The rows of the state one step of the configured solver after (t, yown, v.Y):
+// every lane of the group (all of v.mask) calls it together, and on return all
+// are done reading the state, probes and noise.
+__device__ __forceinline__ void sodecl_lanes_new_state(real_t t, real_t *yown, const sodecl_lanes_view &v, sodecl_i64 gid,
+                                                       double &counter, sodecl_i64 &passes, int &capped, real_t *ynew)
 {
     const real_t h = _m_dt_;
-    real_t ynew[SODECL_ROWS];
 #if SODECL_SOLVER == 1
     // src/kernels/euler.cl:10-18, row by row
 #pragma unroll
@@ -959,8 +1043,13 @@ __device__ __forceinline__ void sodecl_lanes_advance(real_t &t, real_t *yown, co
     (void)counter;
     (void)passes;
     (void)capped;
+    __syncwarp(v.mask);
+}
+
+#ifndef SODECL_SPEC_COPY
+__device__ __forceinline__ void sodecl_lanes_take(real_t &t, real_t *yown, const sodecl_lanes_view &v, const real_t *ynew)
+{
     t = t + _m_dt_;
-    __syncwarp(v.mask);  // the group is done reading the state, probes and noise
 #pragma unroll
     for (int k = 0; k < SODECL_ROWS; ++k) {
         const int r = v.lane + k * SODECL_LANES;
@@ -972,50 +1061,60 @@ __device__ __forceinline__ void sodecl_lanes_advance(real_t &t, real_t *yown, co
     __syncwarp(v.mask);
 }
 
-#ifndef SODECL_SPEC_COPY
-// m steps of the configured solver (m at most SODECL_SPEC_RUN in speculative
-// programs), by every lane of the group together.
+#if SODECL_SPECULATE
+// One lane's flag spoils every row of the orbit, so the group goes by all of its
+// lanes' flags (the ballot's bits of other groups do not count).
+__device__ __forceinline__ bool sodecl_lanes_raised(const sodecl_lanes_view &v)
+{
+    return (__ballot_sync(v.mask, sodecl_raised()) & v.mask) != 0u;
+}
+#endif
+
+// sodecl_advance_run by every lane of the group together.
 __device__ __forceinline__ void sodecl_lanes_advance_run(real_t &t, real_t *yown, const sodecl_lanes_view &v,
                                                          sodecl_i64 gid, double &counter, sodecl_i64 &passes,
-                                                         int &capped, int m)
+                                                         int &capped, sodecl_i64 m)
 {
+    real_t ynew[SODECL_ROWS];
 #if SODECL_SPECULATE
-    const real_t t0 = t;
-    const double counter0 = counter;
-    const sodecl_i64 passes0 = passes;
-    const int capped0 = capped;
-    real_t y0[SODECL_ROWS];
-#pragma unroll
-    for (int k = 0; k < SODECL_ROWS; ++k) y0[k] = yown[k];
+    for (sodecl_i64 q = 0;;) {
+        double c = counter;
 #pragma unroll 1
-    for (int q = 0; q < m; ++q) sodecl_spec::sodecl_lanes_advance(t, yown, v, gid, counter, passes, capped);
-    // one lane's flag spoils every row of the orbit, so the group repeats the
-    // run as one (the ballots' bits of other groups, if any, do not count)
-    if (__ballot_sync(v.mask, sodecl_raised()) & v.mask) {
-        sodecl_lower();
-        bool finite = false;
-#pragma unroll
-        for (int k = 0; k < SODECL_ROWS; ++k)
-            finite = finite || (v.lane + k * SODECL_LANES < _numeq_ && y0[k] == y0[k]);
-        if (__ballot_sync(v.mask, finite) & v.mask) {
-            real_t tc = t0;
-            double cc = counter0;
-            passes = passes0;
-            capped = capped0;
-#pragma unroll
-            for (int k = 0; k < SODECL_ROWS; ++k) {
-                const int r = v.lane + k * SODECL_LANES;
-                yown[k] = y0[k];
-                if (r < _numeq_) v.Y[r] = y0[k];
-            }
-            __syncwarp(v.mask);
-#pragma unroll 1
-            for (int q = 0; q < m; ++q) sodecl_lanes_advance(tc, yown, v, gid, cc, passes, capped);
+        for (; q < m; ++q) {
+            sodecl_i64 n = passes;
+            int cap = capped;
+            sodecl_spec::sodecl_lanes_new_state(t, yown, v, gid, c, n, cap, ynew);
+            if (sodecl_lanes_raised(v)) break;
+            counter = c;
+            passes = n;
+            capped = cap;
+            sodecl_lanes_take(t, yown, v, ynew);
         }
+        if (q >= m) break;
+        bool first = true;
+#pragma unroll 1
+        for (; q < m; ++q) {
+            sodecl_lower();
+            sodecl_i64 n = passes;
+            int cap = capped;
+            c = counter;
+            sodecl_lanes_new_state(t, yown, v, gid, c, n, cap, ynew);
+            const bool up = sodecl_lanes_raised(v);
+            if (!up && !first) break;
+            first = false;
+            counter = c;
+            passes = n;
+            capped = cap;
+            sodecl_lanes_take(t, yown, v, ynew);
+        }
+        sodecl_lower();
     }
 #else
 #pragma unroll 1
-    for (int q = 0; q < m; ++q) sodecl_lanes_advance(t, yown, v, gid, counter, passes, capped);
+    for (sodecl_i64 q = 0; q < m; ++q) {
+        sodecl_lanes_new_state(t, yown, v, gid, counter, passes, capped, ynew);
+        sodecl_lanes_take(t, yown, v, ynew);
+    }
 #endif
 }
 #endif  // SODECL_SPEC_COPY
@@ -1257,6 +1356,7 @@ sodecl_orbits(const sodecl_args a)
                 c = a.chunk_begin;
                 flags = capped = 0;
                 accepted = 0;
+                st.plain = st.tried = false;
                 active = sodecl_dp_open(a, i, c, t, y, p, h, st, flags, accepted, capped);
             }
         }
@@ -1313,13 +1413,7 @@ sodecl_orbits(const sodecl_args a)
     for (int c = a.chunk_begin; c < a.chunk_end; ++c) {
         if (a.records)
             sodecl_store_record(a, c, i, y, flags);
-#if SODECL_SPECULATE
-#pragma unroll 1
-        for (int left = _numsteps_; left > 0; left -= SODECL_SPEC_RUN)
-            sodecl_advance_run(t, y, p, gid, counter, passes, capped, min(SODECL_SPEC_RUN, left));
-#else
         sodecl_advance_run(t, y, p, gid, counter, passes, capped, _numsteps_);
-#endif
     }
     sodecl_orbit_out(a, i, t, y, counter, passes, capped, flags);
 }
@@ -1387,13 +1481,7 @@ sodecl_orbits(const sodecl_args a)
 #pragma unroll 1
     for (int c = a.chunk_begin; c < a.chunk_end; ++c) {
         if (a.records && live) sodecl_lanes_store(a, c, i, yown, lane, flags);
-#if SODECL_SPECULATE
-#pragma unroll 1
-        for (int left = _numsteps_; left > 0; left -= SODECL_SPEC_RUN)
-            sodecl_lanes_advance_run(t, yown, v, gid, counter, passes, capped, min(SODECL_SPEC_RUN, left));
-#else
         sodecl_lanes_advance_run(t, yown, v, gid, counter, passes, capped, _numsteps_);
-#endif
     }
     if (a.write_final && a.records && live) sodecl_lanes_store(a, a.chunk_end, i, yown, lane, flags);
 

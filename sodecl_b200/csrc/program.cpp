@@ -455,8 +455,8 @@ std::vector<std::string> defined_macros(const std::string &src)
 }
 
 // The functions of device/fastmath.cuh in place of the library's, for the
-// copy of the system file that follows: copy is "spec" (the speculative copy)
-// or "full" (the plain one).  The implicit solvers keep the library's exp
+// copy of the system file that follows: copy is "spec" (the speculative copy),
+// "plain" (the one that takes over) or "full" (a program without the two).  The implicit solvers keep the library's exp
 // (fast_math_for).
 std::string math_macros(const std::string &copy, int solver)
 {
@@ -477,6 +477,9 @@ std::string undef_lines(const std::vector<std::string> &names)
     return s;
 }
 
+// Solvers whose speculative programs bring a quotient with each copy
+bool copy_quotients(int solver) { return solver <= 2 || solver == 5; }
+
 // The system file as the solvers see it: with speculative steps its
 // speculative copy first, which with the solvers' step functions lies in a
 // namespace of its own, then the plain copy.
@@ -484,18 +487,19 @@ std::string user_text(const std::string &src, const std::string &name, const std
                       int solver, bool spec_num = false)
 {
     const std::string plain = (as_double.empty() ? "" : "#undef double\n");
-    const std::string spec_double = spec_num ? "typedef sodecl_num real_t;\n#define double sodecl_num\n" : as_double;
     const std::string user = "#line 1 \"" + name + "\"\n" + src + "\n";
     if (math == FastMath::Off) return as_double + user + plain;
+    const bool speculative = math == FastMath::Speculative, quotients = speculative && copy_quotients(solver);
     std::string s;
-    if (math == FastMath::Speculative)
-        s = std::string("namespace sodecl_spec {\n") + (solver <= 2 || solver == 5 ? "SODECL_SPEC_QUOTIENT\n" : "") +
-            spec_double + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_lines(defined_macros(src)) +
+    if (speculative)
+        s = std::string("namespace sodecl_spec {\n") + (quotients ? "SODECL_SPEC_QUOTIENT\n" : "") +
+            (spec_num ? "typedef sodecl_num real_t;\n#define double sodecl_num\n" : as_double) + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_lines(defined_macros(src)) +
             "#ifndef SODECL_STEPS_ONLY\n#define SODECL_STEPS_ONLY 1\n#define SODECL_STEPS_ONLY_HERE 1\n#endif\n"
             "#define SODECL_SPEC_COPY 1\n#line 1 \"solvers.cuh\"\n" + kSolversSrc +
             "\n#undef SODECL_SPEC_COPY\n#ifdef SODECL_STEPS_ONLY_HERE\n#undef SODECL_STEPS_ONLY_HERE\n"
             "#undef SODECL_STEPS_ONLY\n#endif\n}  // namespace sodecl_spec\n";
-    return s + as_double + math_macros("full", solver) + user + undef_math_macros() + plain;
+    return s + (quotients && !spec_num ? "SODECL_PLAIN_QUOTIENT\n" : "") + as_double +
+           math_macros(speculative ? "plain" : "full", solver) + user + undef_math_macros() + plain;
 }
 
 // What a solver can use of device/fastmath.cuh, at most `allowed`.
@@ -509,9 +513,8 @@ std::string user_text(const std::string &src, const std::string &name, const std
 //    quotient are not.  With lanes per orbit the step is a function of its own
 //    and speculates; the one-thread kernel's passes test each argument.
 //  - The adaptive solver accepts steps by an error estimate, and keeps all of
-//    the library's functions; its speculative copy's quotients are the IEEE
-//    quotients.  They need the wrapper, whose plain copy divides as the build
-//    says (speculative_wrapper).
+//    the library's functions; its copies' quotients are the IEEE quotients.  They
+//    need the wrapper (speculative_wrapper).
 //  - FP32: the quotients of the explicit and stochastic solvers with one thread
 //    per orbit, also where the plain copy divides by IEEE division
 //    (speculative_num).  A float's functions are the library's in both copies.
@@ -538,7 +541,7 @@ FastMath fast_math_for(FastMath allowed, const ProgramSpec &s, bool fast_div, co
 }
 
 // Whether a program without the reciprocal quotient goes through sodecl_num all
-// the same, for its speculative copy.
+// the same, for its speculative quotients (the same bits).
 bool speculative_wrapper(const ProgramSpec &s) { return s.solver == 5 && s.fast_math == FastMath::Speculative; }
 
 // Whether the speculative copy alone goes through sodecl_num, the plain copy
@@ -559,8 +562,9 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
     s << "#define SODECL_RECORD_F32 " << (spec.record_f32 ? 1 : 0) << "\n";
     const bool wrapper = spec.fast_div || speculative_wrapper(spec);
     s << "#define SODECL_FAST_DIV " << (wrapper || speculative_num(spec) ? 1 : 0) << "\n";
+    s << "#define SODECL_DIVISION_IEEE " << (spec.fast_div ? 0 : 1) << "\n";
     if (speculative_num(spec)) s << "#define SODECL_SPEC_NUM 1\n";
-    s << "#define SODECL_IEEE_QUOTIENT " << (spec.fast_div ? 0 : 1) << "\n";
+    if (spec.fast_math == FastMath::Speculative && copy_quotients(spec.solver)) s << "#define SODECL_COPY_QUOTIENTS 1\n";
     s << "#define SODECL_HAS_JACOBIAN " << (traits.has_jacobian ? 1 : 0) << "\n";
     s << "#define SODECL_HAS_STOCH " << (traits.has_stoch ? 1 : 0) << "\n";
     s << "#define SODECL_NEWTON_MAX " << spec.newton_max_iter << "\n";
@@ -700,7 +704,7 @@ int reported_bytes(const Program &prog, const char *marker)
 std::shared_ptr<const Program> compile_uncapped(const ProgramSpec &spec, const std::string &system_src,
                                                 const SystemTraits &traits, std::shared_ptr<const Program> capped)
 {
-    if (!spec.liftable_cap || spec.fast_math != FastMath::Speculative ||
+    if (!spec.default_cap || spec.solver != 5 || spec.fast_math != FastMath::Speculative ||
         reported_bytes(*capped, " bytes spill stores") <= 128)
         return capped;
     ProgramSpec free = spec;
@@ -889,6 +893,11 @@ std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string 
             t.fast_div = fast_div;
             t.fast_math = math ? fast_math_for(s.fast_math, s, fast_div, traits, system_src) : FastMath::Off;
             if (math && t.fast_math == FastMath::Off) continue;
+            // RK4 in FP64: with the straight-line functions' constants and both
+            // copies, 85 registers spill within the step (oculomotor, 2^20 orbits x
+            // 1000 steps: 31.6 ms so, 28.7 at 128 registers)
+            if (t.default_cap && t.solver == 2 && t.fast_math == FastMath::Speculative)
+                t.min_blocks = std::max(1, 65536 / (t.block_max * 128));
             if (!fast_div && !math) return compile_one(t, system_src, traits);
             try {
                 return compile_uncapped(t, system_src, traits, compile_one(t, system_src, traits));

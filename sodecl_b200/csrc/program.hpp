@@ -27,7 +27,7 @@ struct ProgramSpec {
     bool fp32 = false;
     bool fmad = true;
     bool record_f32 = false;
-    bool liftable_cap = false;  // min_blocks is a default that may go (build)
+    bool default_cap = false;   // min_blocks is a default, for programs without speculative steps (build)
     bool fast_div = false;   // FP64 through sodecl_f64 (exact reciprocal quotients)
     double newton_tol = 1e-7;
     int newton_max_iter = 1000;

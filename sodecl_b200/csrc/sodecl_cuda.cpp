@@ -538,7 +538,7 @@ ProgramSpec make_spec(const sodecl_cfg &c)
         (c.solver == SODECL_IMPLICIT_EULER || c.solver == SODECL_IMPLICIT_MIDPOINT ||
          c.solver == SODECL_DORMAND_PRINCE)) {
         spec.min_blocks = std::max(1, 65536 / (spec.block_max * 128));
-        spec.liftable_cap = c.solver == SODECL_DORMAND_PRINCE;
+        spec.default_cap = c.solver == SODECL_DORMAND_PRINCE;
     }
     // FP64 RK4 on small systems, one thread per orbit: by default at most 85
     // registers a thread (three blocks of 256).  Measured on the oculomotor
@@ -546,8 +546,10 @@ ProgramSpec make_spec(const sodecl_cfg &c)
     // and 411 ms at 64 registers (the reference's system file; the package's
     // 362 / 381 / 371 ms).
     if (spec.min_blocks == 0 && lanes_of(c) == 1 && c.solver == SODECL_RUNGE_KUTTA && !spec.fp32 &&
-        c.num_equat <= 8)
+        c.num_equat <= 8) {
         spec.min_blocks = std::max(1, 65536 / (spec.block_max * 85));
+        spec.default_cap = true;
+    }
     spec.fast_div = reciprocal_division(c);
     spec.lanes = lanes_of(c);
     // sin, cos, exp and quotients without branches

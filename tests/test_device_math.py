@@ -104,15 +104,14 @@ def check_quotients(name, a, b, covered):
     assert np.isnan(q[inside & nan]).all()
     same = inside & ~nan
     np.testing.assert_array_equal(q[same].view(word), want[same].view(word))
-    assert not outside[nan & (np.isnan(a) | np.isnan(b)) & covered].any()
-    assert not outside[covered & ~nan].any()
+    assert not outside[covered].any()
 
 
 @pytest.mark.parametrize("name", ["chain", "straight"])
 def test_quotients_have_the_ieee_quotients_bits(name):
     a, b = pairs(53, 2000000, 4)
     with np.errstate(all="ignore"):
-        moderate = ((np.abs(a) > 1e-20) & (np.abs(a) < 1e40) | ((a == 0) & ~np.signbit(a)) | np.isnan(a)) & \
+        moderate = ((np.abs(a) > 1e-20) & (np.abs(a) < 1e40) | ((a == 0) & ~np.signbit(a))) & \
             (np.abs(b) > 1e-20) & (np.abs(b) < 1e28) & (np.frexp(np.abs(b))[0] != 1 - 2.0 ** -53)
     check_quotients(name + "_quotients", a, b, moderate)
 
@@ -121,5 +120,5 @@ def test_float_quotients_have_the_ieee_quotients_bits():
     a, b = pairs(24, 2000000, 5)
     a = np.concatenate([a, np.float32([float.fromhex("0x1.d074d8p+0")])])
     b = np.concatenate([b, np.float32([float.fromhex("0x1.527e7cp+0")])])
-    moderate = ((np.abs(a) > 1e-20) & (np.abs(a) < 1e20) | ((a == 0) & ~np.signbit(a)) | np.isnan(a)) & (np.abs(b) > 1e-10) & (np.abs(b) < 1e10)
+    moderate = ((np.abs(a) > 1e-30) & (np.abs(a) < 1e30) | ((a == 0) & ~np.signbit(a))) & (np.abs(b) > 1e-7) & (np.abs(b) < 1e7)
     check_quotients("straight_quotients_f32", a, b, moderate)
