@@ -537,7 +537,9 @@ FastMath fast_math_for(FastMath allowed, const ProgramSpec &s, bool fast_div, co
     if (s.solver == 5) return s.num_equat <= 256 ? allowed : FastMath::Off;
     const bool quotient = t.uses_division || s.solver == 2;
     const bool gain = s.fp32 ? quotient : t.uses_trig || t.uses_exp || (fast_div && quotient);
-    return gain && (s.lanes > 1 || s.num_equat <= 256) ? allowed : FastMath::Off;
+    if (!gain) return FastMath::Off;
+    if (s.lanes > 1 || s.num_equat <= 256) return allowed;
+    return !s.fp32 && (t.uses_trig || t.uses_exp) ? FastMath::Guarded : FastMath::Off;  // the lanes' values
 }
 
 // Whether a program without the reciprocal quotient goes through sodecl_num all

@@ -142,3 +142,14 @@ def test_such_files_in_fp32_lanes_and_batches(tmp_path):
 def test_shipped_systems_keep_it(system):
     with open(system_path(system)) as f:
         assert speculates(f.read(), neq=6, npar=7)
+
+
+@pytest.mark.parametrize("neq,copies", [(256, 2), (257, 1)])
+def test_wide_systems_take_the_same_functions(neq, copies):
+    """One thread per orbit and lanes per orbit get the same sines, whatever the
+    number of equations (one thread's steps speculate up to 256)."""
+    with open(system_path("kuramoto")) as f:
+        source = f.read()
+    for lanes in (1, 32):
+        with Integrator(None, "euler", system_src=source, dt=0.1, tspan=1.0, ksteps=1, neq=neq, npar=neq + 1, orbits=1, lanes=lanes) as sim:
+            assert sim.program_source.count("#define sin(...)") == (copies if lanes == 1 else 2)

@@ -163,3 +163,16 @@ def test_implicit_steps_beyond_the_sines_range(solver):
             out.append((sim.run(), *sim.status()))
     for one, many in zip(*out):
         np.testing.assert_array_equal(many, one)
+
+
+def test_one_thread_and_lanes_agree_beyond_256_equations():
+    n, neq = 3, 260
+    rng = np.random.default_rng(9)
+    y0, p = rng.uniform(0, 6, (n, neq)), np.concatenate([np.full((n, 1), 2.0), rng.normal(size=(n, neq))], axis=1)
+    out = []
+    for lanes in (1, 32):
+        with Integrator(system_path("kuramoto"), "euler", dt=0.01, tspan=0.045, ksteps=2, neq=neq, npar=neq + 1, orbits=n,
+                        lanes=lanes, fmad=False) as sim:
+            sim.upload(np.zeros(n), y0, p)
+            out.append(sim.run())
+    np.testing.assert_array_equal(*out)
