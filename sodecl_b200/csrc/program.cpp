@@ -17,6 +17,7 @@
 #include <sys/stat.h>
 #include <unistd.h>
 
+#include <algorithm>
 #include <cctype>
 #include <cmath>
 #include <cstdint>
@@ -442,16 +443,48 @@ int lanes_slot_words(const ProgramSpec &spec)
 
 namespace {
 
-// Names of the object-like and function-like macros a source #defines, so a
-// batch program can #undef them after each class.
+// The names a source #defines, wherever they stand, each once.
 std::vector<std::string> defined_macros(const std::string &src)
 {
     std::vector<std::string> names;
-    const std::regex def("^[ \\t]*#[ \\t]*define[ \\t]+([A-Za-z_][A-Za-z0-9_]*)");
-    const std::string stripped = scan_code(src, [](const std::string &x) { return x; }, false);
-    for (std::sregex_iterator it(stripped.begin(), stripped.end(), def), end; it != end; ++it)
-        names.push_back((*it)[1].str());
+    const std::string code = scan_code(src, [](const std::string &x) { return x; }, false);
+    const auto skip = [&](size_t i) {
+        while (i < code.size() && (code[i] == ' ' || code[i] == '\t')) ++i;
+        return i;
+    };
+    for (size_t line = 0; line < code.size();) {
+        size_t i = skip(line);
+        line = code.find('\n', line);
+        line = line == std::string::npos ? code.size() : line + 1;
+        if (i >= code.size() || code[i] != '#') continue;
+        i = skip(i + 1);
+        if (code.compare(i, 6, "define") != 0 || i + 6 >= code.size() || ident_char(code[i + 6])) continue;
+        i = skip(i + 6);
+        size_t j = i;
+        while (j < code.size() && ident_char(code[j])) ++j;
+        const std::string name = code.substr(i, j - i);
+        if (!name.empty() && std::find(names.begin(), names.end(), name) == names.end()) names.push_back(name);
+    }
     return names;
+}
+
+// A system file compiled a second time, or behind another one, has to find no
+// macro that its first copy (the other file) left: a helper within
+// `#ifndef X / #define X / #endif` would be missing.  What was defined before
+// stays (`#ifndef M_PI / #define M_PI 3.14 / #endif` leaves the program's M_PI
+// alone).  Before and after the text:
+std::string note_macros(const std::vector<std::string> &names)
+{
+    std::string s;
+    for (const auto &n : names)
+        s += "#undef SODECL_HAD_" + n + "\n#ifdef " + n + "\n#define SODECL_HAD_" + n + "\n#endif\n";
+    return s;
+}
+std::string undef_macros(const std::vector<std::string> &names)
+{
+    std::string s;
+    for (const auto &n : names) s += "#ifndef SODECL_HAD_" + n + "\n#undef " + n + "\n#endif\n";
+    return s;
 }
 
 // The functions of device/fastmath.cuh in place of the library's, for the
@@ -470,13 +503,6 @@ std::string math_macros(const std::string &copy, int solver)
 
 std::string undef_math_macros() { return "#undef sin\n#undef cos\n#undef exp\n#undef sincos\n"; }
 
-std::string undef_lines(const std::vector<std::string> &names)
-{
-    std::string s;
-    for (const auto &n : names) s += "#undef " + n + "\n";
-    return s;
-}
-
 // Solvers whose speculative programs bring a quotient with each copy
 bool copy_quotients(int solver) { return solver <= 2 || solver == 5; }
 
@@ -493,7 +519,7 @@ std::string user_text(const std::string &src, const std::string &name, const std
     std::string s;
     if (speculative)
         s = std::string("namespace sodecl_spec {\n") + (quotients ? "SODECL_SPEC_QUOTIENT\n" : "") +
-            (spec_num ? "typedef sodecl_num real_t;\n#define double sodecl_num\n" : as_double) + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_lines(defined_macros(src)) +
+            note_macros(defined_macros(src)) + (spec_num ? "typedef sodecl_num real_t;\n#define double sodecl_num\n" : as_double) + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_macros(defined_macros(src)) +
             "#ifndef SODECL_STEPS_ONLY\n#define SODECL_STEPS_ONLY 1\n#define SODECL_STEPS_ONLY_HERE 1\n#endif\n"
             "#define SODECL_SPEC_COPY 1\n#line 1 \"solvers.cuh\"\n" + kSolversSrc +
             "\n#undef SODECL_SPEC_COPY\n#ifdef SODECL_STEPS_ONLY_HERE\n#undef SODECL_STEPS_ONLY_HERE\n"
@@ -559,6 +585,7 @@ std::string assemble(const ProgramSpec &spec, const std::string &system_src, con
 {
     std::ostringstream s;
     s << "// SODECL program generated by libsodecl_cuda (sm_100a)\n";
+    if (!spec.plain_why.empty()) s << "// no speculative copy: " << spec.plain_why << "\n";
     s << "#define SODECL_SOLVER " << spec.solver << "\n";
     s << "#define SODECL_FP32 " << (spec.fp32 ? 1 : 0) << "\n";
     s << "#define SODECL_RECORD_F32 " << (spec.record_f32 ? 1 : 0) << "\n";
@@ -674,6 +701,16 @@ std::shared_ptr<const Program> compile_text(std::string source, bool fmad, bool 
     return done;
 }
 
+// The first error of a failed compilation, as one line of a comment.
+std::string first_error(const std::string &message)
+{
+    size_t at = message.find("error:");
+    if (at == std::string::npos) at = 0;
+    std::string line = message.substr(at, message.find('\n', at) - at);
+    if (!line.empty() && line.back() == '\\') line.pop_back();
+    return "it did not compile with one (" + line + ")";
+}
+
 std::shared_ptr<const Program> compile_one(const ProgramSpec &spec, const std::string &system_src,
                                            const SystemTraits &traits)
 {
@@ -730,10 +767,11 @@ int batch_warp_words(const std::vector<BatchClass> &classes)
 namespace {
 
 std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div, FastMath allowed, int block_max,
-                           int min_blocks)
+                           int min_blocks, const std::string &why)
 {
     std::ostringstream s;
     s << "// SODECL batch program generated by libsodecl_cuda (sm_100a)\n";
+    if (!why.empty()) s << "// no speculative copy: " << why << "\n";
     s << "#define SODECL_STEPS_ONLY 1\n#define SODECL_FP32 0\n#define SODECL_RECORD_F32 0\n";
     s << "#define SODECL_FAST_DIV " << (fast_div ? 1 : 0) << "\n";
     s << "#define SODECL_BLOCK_MAX " << block_max << "\n";
@@ -752,6 +790,7 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
         const SystemTraits tr = inspect_system(src);
         const FastMath math = fast_math_for(allowed, sp, fast_div, tr, src);
         s << "\n// ---- class " << k << "\n";
+        if (!tr.speculation_hazard.empty()) s << "// no speculative copy: " << tr.speculation_hazard << "\n";
         for (const char *m : per_class) s << "#undef " << m << "\n";
         s << "#define SODECL_SOLVER " << sp.solver << "\n";
         s << "#define SODECL_HAS_JACOBIAN " << (tr.has_jacobian ? 1 : 0) << "\n";
@@ -771,10 +810,11 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
         s << "#define _numpar_ " << sp.num_params << "\n";
         s << "#define _epsilon1_ " << print_like_reference(sp.newton_tol) << "\n";
         s << l2_bound_define(sp.newton_tol, false);
-        s << "namespace sodecl_cls_" << k << " {\n";
+        const std::vector<std::string> macros = defined_macros(src);
+        s << note_macros(macros) << "namespace sodecl_cls_" << k << " {\n";
         s << user_text(relax_parameter_bounds(src), "class" + std::to_string(k) + ".cl",
                        fast_div ? "#define double sodecl_num\n" : "", math, sp.solver);
-        for (const auto &m : defined_macros(src)) s << "#undef " << m << "\n";
+        s << undef_macros(macros);
         s << "#line 1 \"solvers.cuh\"\n" << kSolversSrc << "\n";
         s << "#define SODECL_BATCH_CLASS_BODY 1\n#line 1 \"batch.cuh\"\n" << kBatchSrc << "\n";
         s << "}  // namespace sodecl_cls_" << k << "\n";
@@ -864,14 +904,17 @@ std::shared_ptr<const Program> build_batch(const std::vector<BatchClass> &classe
     for (const auto &c : classes)
         if (c.system_src.find("printf") != std::string::npos) fd = false;
     // as for one system: the plainer programs where a system file needs them
+    std::string why;
     for (const bool div : {true, false}) {
         for (const FastMath math : {FastMath::Speculative, FastMath::Off}) {
             if (div && !fd) continue;
-            const std::string text = assemble_batch(classes, div, math, block_max, min_blocks);
+            const std::string text = assemble_batch(classes, div, math, block_max, min_blocks,
+                                                    math == FastMath::Off ? why : std::string());
             if (!div && math == FastMath::Off) return compile_text(text, fmad, div, "sodecl_batch");
             try {
                 return compile_text(text, fmad, div, "sodecl_batch", math != FastMath::Off);
-            } catch (const std::exception &) {
+            } catch (const std::exception &e) {
+                if (math != FastMath::Off) why = first_error(e.what());
             }
         }
     }
@@ -888,6 +931,7 @@ std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string 
     // does not compile with the wrapper, and one that declares or redefines
     // the math functions does not with fastmath.cuh's: the next plainer
     // program is built instead, the division mode kept as long as it can be
+    std::string why;
     for (const bool fast_div : {true, false}) {
         if (fast_div && !s.fast_div) continue;
         for (const bool math : {true, false}) {
@@ -895,6 +939,7 @@ std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string 
             t.fast_div = fast_div;
             t.fast_math = math ? fast_math_for(s.fast_math, s, fast_div, traits, system_src) : FastMath::Off;
             if (math && t.fast_math == FastMath::Off) continue;
+            t.plain_why = t.fast_math == FastMath::Speculative ? "" : !why.empty() ? why : traits.speculation_hazard;
             // RK4 in FP64: with the straight-line functions' constants and both
             // copies, 85 registers spill within the step (oculomotor, 2^20 orbits x
             // 1000 steps: 31.6 ms so, 28.7 at 128 registers)
@@ -903,7 +948,8 @@ std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string 
             if (!fast_div && !math) return compile_one(t, system_src, traits);
             try {
                 return compile_uncapped(t, system_src, traits, compile_one(t, system_src, traits));
-            } catch (const std::exception &) {
+            } catch (const std::exception &e) {
+                if (math) why = first_error(e.what());
             }
         }
     }

@@ -35,6 +35,7 @@ struct ProgramSpec {
     int min_blocks = 0;
     int lanes = 1;           // lanes per orbit (1, or a power of two up to 32)
     FastMath fast_math = FastMath::Off;
+    std::string plain_why;   // why it is not what fast_math allowed, for the program text
     bool pair_stores = false;  // one thread per orbit: records two orbits per vector store
     double rtol = 1e-6;      // adaptive solver (solver 5): error tolerances and
     double atol = 1e-9;      // step attempts per record interval

@@ -153,3 +153,31 @@ def test_wide_systems_take_the_same_functions(neq, copies):
     for lanes in (1, 32):
         with Integrator(None, "euler", system_src=source, dt=0.1, tspan=1.0, ksteps=1, neq=neq, npar=neq + 1, orbits=1, lanes=lanes) as sim:
             assert sim.program_source.count("#define sin(...)") == (copies if lanes == 1 else 2)
+
+
+GUARDED = "/* helpers */\n#ifndef X_CL\n#define X_CL\n#ifndef M_PI\n  #  define M_PI 3.0\n#endif\n#define GAIN 2.0\n" \
+    "static_assert(M_PI > 3.1);\ndouble f(double x) { return GAIN * sin(M_PI * x); }\n" + HEAD + \
+    "\tyout[0] = f(y[0]) / p[0];\n}\n#endif\n"
+
+
+def test_guarded_files_keep_it():
+    """Neither copy, nor a second class of a batch, finds what the first one defined;
+    what the program defines stays."""
+    assert speculates(GUARDED)
+    b = Batch()
+    for solver in ("euler", "rk4"):
+        b.add_class(None, solver, neq=1, npar=1, dt=0.1, system_src=GUARDED)
+    text = b.compile().program_source
+    assert text.count("#define SODECL_SPECULATE 1") == 2 and "no speculative copy" not in text
+
+
+def test_the_reason_for_no_copy_is_in_the_program():
+    def reason(source):
+        with Integrator(None, "rk4", system_src=source, dt=0.1, tspan=1.0, ksteps=1, neq=3, npar=12, orbits=1) as sim:
+            lines = [line for line in sim.program_source.splitlines() if line.startswith("// no speculative copy: ")]
+            assert len(lines) == (0 if "#define SODECL_SPECULATE 1" in sim.program_source else 1)
+            return lines[0] if lines else ""
+
+    assert reason(SAFE["plain"]) == ""
+    assert reason(HEAD + HAZARDS["while"] + "}\n").endswith(": while")
+    assert "did not compile" in reason("double sin(double x) { return x; }\n" + HEAD + "\tyout[0] = sin(y[0]);\n}\n")
