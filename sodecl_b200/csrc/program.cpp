@@ -405,7 +405,8 @@ SystemTraits inspect_system(const std::string &src)
 {
     const std::string stripped = scan_code(src, [](const std::string &s) { return s; }, false);
     SystemTraits t;
-    t.uses_division = stripped.find('/') != std::string::npos;
+    t.quotients = static_cast<int>(std::count(stripped.begin(), stripped.end(), '/'));
+    t.uses_division = t.quotients > 0;
     t.speculation_hazard = speculation_hazard(stripped);
     const std::pair<std::string_view, bool *> functions[] = {
         {"sode_system", &t.has_system},
@@ -422,8 +423,18 @@ SystemTraits inspect_system(const std::string &src)
         if (word == "_listsize_") t.uses_listsize = true;
         const size_t open = open_parenthesis(stripped, end);
         if (open == std::string::npos) return;
-        for (const auto &f : functions)
-            if (word == f.first && !*f.second) *f.second = definition_follows(stripped, open);
+        for (const auto &f : functions) {
+            if (word != f.first || *f.second || !definition_follows(stripped, open)) continue;
+            *f.second = true;
+            if (f.second == &t.has_system) continue;
+            // the other hooks' bodies are not part of a right-hand side
+            size_t body = stripped.find('{', open), depth = 0;
+            for (; body < stripped.size(); ++body) {
+                if (stripped[body] == '{') ++depth;
+                if (stripped[body] == '/') --t.quotients;
+                if (stripped[body] == '}' && --depth == 0) break;
+            }
+        }
         for (const std::string_view prefix : {"native_", "half_"})
             if (word.substr(0, prefix.size()) == prefix) {
                 word.remove_prefix(prefix.size());
@@ -528,6 +539,20 @@ std::string user_text(const std::string &src, const std::string &name, const std
            math_macros(speculative ? "plain" : "full", solver) + user + undef_math_macros() + plain;
 }
 
+// Orbits up to which the adaptive solver speculates: twice what its plain kernel
+// (128 registers) holds on a B200 at once, 2 x 148 x 512.  Up to there a launch
+// waits for its longest chains of attempts; beyond, throughput counts, and the
+// registers of the speculative attempt's reciprocals cost more occupancy than its
+// straight-line quotients save.  Oculomotor, speculative against plain: over 0.02
+// time units 12.0 / 14.9 ms at 4097 orbits, 27.5 / 32.0 at 2^17, 107 / 92 at 2^20;
+// over 0.2 units 38.8 / 44.4 at 2^14, 74.3 / 75.3 at 2^17, 285 / 240 at 2^20.
+constexpr int64_t kLatencyOrbits = 2 * 148 * 512;
+// The same for files with fewer quotients than equations, whose attempts the
+// library's functions make: Kuramoto of 3, 5 and 9 phases 0.38 / 0.36, 1.58 / 1.26 and
+// 3.44 / 3.40 ms at 1024 orbits.  Two warps' launches (0.33 / 0.32, 1.16 / 0.87, 3.12 /
+// 3.09 ms) end within the host work of a call either way.
+constexpr int64_t kFewOrbits = 64;
+
 // What a solver can use of device/fastmath.cuh, at most `allowed`.
 //  - Euler, RK4 and Euler-Maruyama evaluate a fixed sequence: speculative steps
 //    wherever a function or a reciprocal quotient is called (RK4 divides by
@@ -539,7 +564,8 @@ std::string user_text(const std::string &src, const std::string &name, const std
 //    quotient are not.  With lanes per orbit the step is a function of its own
 //    and speculates; the one-thread kernel's passes test each argument.
 //  - The adaptive solver accepts steps by an error estimate, and keeps all of
-//    the library's functions; its copies' quotients are the IEEE quotients.  They
+//    the library's functions; its copies' quotients are the IEEE quotients, for
+//    launches that wait for latency (kLatencyOrbits).  They
 //    need the wrapper (speculative_wrapper).
 //  - FP32: the quotients of the explicit and stochastic solvers with one thread
 //    per orbit, also where the plain copy divides by IEEE division
@@ -560,7 +586,9 @@ FastMath fast_math_for(FastMath allowed, const ProgramSpec &s, bool fast_div, co
         return s.lanes > 1 && safe ? allowed : FastMath::Guarded;
     }
     if (!safe) return FastMath::Off;
-    if (s.solver == 5) return s.num_equat <= 256 ? allowed : FastMath::Off;
+    if (s.solver == 5)
+        return s.num_equat <= 256 && s.list_size <= (t.quotients >= s.num_equat ? kLatencyOrbits : kFewOrbits) ? allowed
+                                                                                                              : FastMath::Off;
     const bool quotient = t.uses_division || s.solver == 2;
     const bool gain = s.fp32 ? quotient : t.uses_trig || t.uses_exp || (fast_div && quotient);
     if (!gain) return FastMath::Off;
@@ -732,14 +760,16 @@ int reported_bytes(const Program &prog, const char *marker)
 }
 
 // `capped`, or the program without the register cap where only that keeps
-// everything in registers.  Attempts of the adaptive solver are one long chain
-// for each lane, so their latency counts as much as occupancy: the oculomotor
-// model over 0.02 time units took 12.0 ms without the cap (228 registers)
-// against 15.1 with it at 4097 orbits, 25.2 against 32.7 at 2^17, 88 against
-// 98 at 2^20, Kuramoto of 5 phases 4.1 against 7.5 at 2^17.  Where the cap
-// spills next to nothing, or the state stays in local memory all the same (a
-// slow path of the math library keeps 40 bytes there), occupancy is worth more
-// (Kuramoto at 2^17: 3 phases 1.47 against 2.20 ms, 8 phases 17 against 22).
+// everything in registers.  The attempts of the adaptive solver's speculative
+// program (few orbits: kLatencyOrbits) are one long chain for each lane, so what
+// spills on it counts and occupancy hardly: oculomotor 12.0 ms without the cap (222
+// registers) against 15.5 with it (542 bytes spilt) at 4097 orbits over 0.02 time
+// units, 38.8 against 50.6 at 2^14 over 0.2, 74.3 against 83.8 at 2^17.  Up to 128
+// bytes, some 16 of the cap's 128 registers, stay in the first-level cache next to
+// the chain's quotients and occupancy is worth as much (Kuramoto of 5 phases, 16
+// bytes: 1.30 with the cap, 1.24 without at 2^14 orbits, 3.35 and 3.94 at 2^17);
+// and where the uncapped program keeps more than the math library's slow path in
+// local memory all the same (40 bytes), the state is not in registers either.
 std::shared_ptr<const Program> compile_uncapped(const ProgramSpec &spec, const std::string &system_src,
                                                 const SystemTraits &traits, std::shared_ptr<const Program> capped)
 {

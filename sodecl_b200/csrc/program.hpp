@@ -64,6 +64,7 @@ struct SystemTraits {
     bool has_vjp = false;        // calc_vjp (v^T df/dy and v^T df/dp), used by the adjoint
     bool uses_listsize = false;
     bool uses_division = false;
+    int quotients = 0;           // divisions in sode_system and the file's helpers
     bool uses_trig = false;      // calls sin, cos or sincos, and
     bool uses_exp = false;       // exp (the functions of device/fastmath.cuh)
     std::string speculation_hazard;  // why it gets no speculative copy (speculable.hpp), or empty

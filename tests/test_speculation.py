@@ -181,3 +181,17 @@ def test_the_reason_for_no_copy_is_in_the_program():
     assert reason(SAFE["plain"]) == ""
     assert reason(HEAD + HAZARDS["while"] + "}\n").endswith(": while")
     assert "did not compile" in reason("double sin(double x) { return x; }\n" + HEAD + "\tyout[0] = sin(y[0]);\n}\n")
+
+
+def test_the_adaptive_solver_speculates_for_few_orbits():
+    """Up to twice the threads that its plain kernel keeps on the device (2 x 148 x
+    512) where the file has a quotient for every equation, else up to two warps."""
+    with open(system_path("oculomotor")) as f:
+        source = f.read()
+    assert speculates(source, "dp45", neq=6, npar=6, orbits=2 * 148 * 512)
+    assert not speculates(source, "dp45", neq=6, npar=6, orbits=2 * 148 * 512 + 1)
+    assert speculates(source, "rk4", neq=6, npar=6, orbits=1 << 20)
+    with open(system_path("kuramoto")) as f:
+        source = f.read()
+    # one quotient for all rows
+    assert speculates(source, "dp45", neq=5, npar=6, orbits=64) and not speculates(source, "dp45", neq=5, npar=6, orbits=65)

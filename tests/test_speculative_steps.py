@@ -176,3 +176,22 @@ def test_one_thread_and_lanes_agree_beyond_256_equations():
             sim.upload(np.zeros(n), y0, p)
             out.append(sim.run())
     np.testing.assert_array_equal(*out)
+
+
+@pytest.mark.parametrize("system,neq,dt", [("kuramoto", 5, 0.01), ("oculomotor", 6, 1e-4)])
+def test_adaptive_steps_with_contraction(system, neq, dt):
+    """Few orbits take the speculative program, many the plain one: the same
+    attempts and records with FMA contraction too."""
+    with open(system_path(system)) as f:
+        source = f.read()
+    n = 777 if system == "oculomotor" else 60
+    rng = np.random.default_rng(neq)
+    if system == "kuramoto":
+        p = np.concatenate([rng.uniform(0, 5, (n, 1)), rng.normal(size=(n, neq))], axis=1)
+        y0 = rng.uniform(0, 2 * np.pi, (n, neq))
+    else:
+        p = np.array([120.0, 1.5, 0.0045, 0.05, 600.0, 9.0]) * rng.uniform(0.5, 1.5, (n, 6))
+        y0 = np.tile([0.0, 0.0, 0.0, 0.0, 0.0, 2.0], (n, 1)) * rng.uniform(0.5, 1.5, (n, 1))
+    got, plain = run(source, "dp45", y0, p, dt=dt, tspan=199.5 * dt, ksteps=20, fmad=True)
+    for a, b in zip(got, plain):
+        np.testing.assert_array_equal(a, b)
