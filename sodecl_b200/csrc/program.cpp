@@ -401,13 +401,23 @@ std::string suffix_float_literals(const std::string &src)
     return scan_code(src, suffix_in_code, true);
 }
 
+namespace {
+// The traits of a file that is about to be compiled: speculation_hazard too,
+// which takes longer than the rest.
+SystemTraits inspect_for_build(const std::string &src)
+{
+    SystemTraits t = inspect_system(src);
+    t.speculation_hazard = speculation_hazard(scan_code(src, [](const std::string &s) { return s; }, false));
+    return t;
+}
+}  // namespace
+
 SystemTraits inspect_system(const std::string &src)
 {
     const std::string stripped = scan_code(src, [](const std::string &s) { return s; }, false);
     SystemTraits t;
     t.quotients = static_cast<int>(std::count(stripped.begin(), stripped.end(), '/'));
     t.uses_division = t.quotients > 0;
-    t.speculation_hazard = speculation_hazard(stripped);
     const std::pair<std::string_view, bool *> functions[] = {
         {"sode_system", &t.has_system},
         {"calc_jacobian", &t.has_jacobian},
@@ -526,11 +536,12 @@ std::string user_text(const std::string &src, const std::string &name, const std
     const std::string plain = (as_double.empty() ? "" : "#undef double\n");
     const std::string user = "#line 1 \"" + name + "\"\n" + src + "\n";
     if (math == FastMath::Off) return as_double + user + plain;
+    const std::vector<std::string> macros = math == FastMath::Speculative ? defined_macros(src) : std::vector<std::string>();
     const bool speculative = math == FastMath::Speculative, quotients = speculative && copy_quotients(solver);
     std::string s;
     if (speculative)
         s = std::string("namespace sodecl_spec {\n") + (quotients ? "SODECL_SPEC_QUOTIENT\n" : "") +
-            note_macros(defined_macros(src)) + (spec_num ? "typedef sodecl_num real_t;\n#define double sodecl_num\n" : as_double) + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_macros(defined_macros(src)) +
+            note_macros(macros) + (spec_num ? "typedef sodecl_num real_t;\n#define double sodecl_num\n" : as_double) + math_macros("spec", solver) + user + undef_math_macros() + plain + undef_macros(macros) +
             "#ifndef SODECL_STEPS_ONLY\n#define SODECL_STEPS_ONLY 1\n#define SODECL_STEPS_ONLY_HERE 1\n#endif\n"
             "#define SODECL_SPEC_COPY 1\n#line 1 \"solvers.cuh\"\n" + kSolversSrc +
             "\n#undef SODECL_SPEC_COPY\n#ifdef SODECL_STEPS_ONLY_HERE\n#undef SODECL_STEPS_ONLY_HERE\n"
@@ -817,7 +828,7 @@ std::string assemble_batch(const std::vector<BatchClass> &classes, bool fast_div
     for (size_t k = 0; k < classes.size(); ++k) {
         const ProgramSpec &sp = classes[k].spec;
         const std::string &src = classes[k].system_src;
-        const SystemTraits tr = inspect_system(src);
+        const SystemTraits tr = inspect_for_build(src);
         const FastMath math = fast_math_for(allowed, sp, fast_div, tr, src);
         s << "\n// ---- class " << k << "\n";
         if (!tr.speculation_hazard.empty()) s << "// no speculative copy: " << tr.speculation_hazard << "\n";
@@ -953,7 +964,7 @@ std::shared_ptr<const Program> build_batch(const std::vector<BatchClass> &classe
 
 std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string &system_src)
 {
-    const SystemTraits traits = inspect_system(system_src);
+    const SystemTraits traits = inspect_for_build(system_src);
     ProgramSpec s = spec;
     // the wrapper type would hand a struct to printf's varargs
     if (system_src.find("printf") != std::string::npos) s.fast_div = false;

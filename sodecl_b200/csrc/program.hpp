@@ -67,7 +67,7 @@ struct SystemTraits {
     int quotients = 0;           // divisions in sode_system and the file's helpers
     bool uses_trig = false;      // calls sin, cos or sincos, and
     bool uses_exp = false;       // exp (the functions of device/fastmath.cuh)
-    std::string speculation_hazard;  // why it gets no speculative copy (speculable.hpp), or empty
+    std::string speculation_hazard;  // why it gets no speculative copy (speculable.hpp); filled for a build
 };
 
 SystemTraits inspect_system(const std::string &src);

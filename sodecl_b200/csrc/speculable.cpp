@@ -3,6 +3,8 @@
 #include <cctype>
 #include <map>
 #include <set>
+#include <string_view>
+#include <unordered_map>
 #include <vector>
 
 namespace sodecl_b200 {
@@ -11,23 +13,62 @@ namespace {
 
 enum class Kind { Ident, Number, Punct };
 
+// The scan runs on every compilation and gradient call, so a word is looked up
+// once, when it is read.
+enum Class : unsigned char { kPlain = 0, kIntType = 1, kRefusedWord = 2, kKeyword = 4 };
+
 struct Tok {
     Kind kind;
-    std::string text;
+    std::string_view text;
+    unsigned char cls = kPlain;
 };
 
 using Toks = std::vector<Tok>;
-using Names = std::set<std::string>;
+using Names = std::set<std::string_view>;
 
 bool ident_start(char c) { return std::isalpha(static_cast<unsigned char>(c)) || c == '_'; }
 bool ident_char(char c) { return std::isalnum(static_cast<unsigned char>(c)) || c == '_'; }
 
+const std::string_view kIntTypes[] = {"int",   "unsigned", "signed", "long",   "short",    "char",      "size_t",   "ptrdiff_t",
+                         "uint",  "ulong",    "ushort", "uchar",  "intptr_t", "uintptr_t", "int8_t",   "int16_t",
+                         "int32_t", "int64_t", "uint8_t", "uint16_t", "uint32_t", "uint64_t", "wchar_t"};
+
+const std::string_view kRefused[] = {"while",    "do",      "goto",  "switch",   "asm",       "__asm",    "__asm__",  "printf",
+                        "template", "union",   "enum",  "typedef",  "using",     "namespace", "class",   "struct",
+                        "auto",     "decltype", "typeof", "__typeof__", "operator", "new",    "delete",   "malloc",
+                        "free",     "try",     "throw", "volatile", "reinterpret_cast", "const_cast", "__builtin_assume",
+                        "sizeof",   "alignof", "extern", "__trap", "__syncthreads", "__syncwarp"};
+
+bool vector_of_ints(std::string_view w)  // int2, uchar4, longlong2, ...
+{
+    if (w.size() < 4 || !std::isdigit(static_cast<unsigned char>(w.back()))) return false;
+    size_t n = w.size();
+    while (n > 0 && std::isdigit(static_cast<unsigned char>(w[n - 1]))) --n;
+    std::string_view base = w.substr(0, n);
+    if (!base.empty() && base[0] == 'u') base.remove_prefix(1);
+    return base == "int" || base == "long" || base == "longlong" || base == "short" || base == "char";
+}
+
+unsigned char class_of(std::string_view w)
+{
+    static const std::unordered_map<std::string_view, unsigned char> words = [] {
+        std::unordered_map<std::string_view, unsigned char> m;
+        for (const auto t : kIntTypes) m[t] = kIntType;
+        for (const auto t : kRefused) m[t] = kRefusedWord;
+        for (const std::string_view t : {"double", "float", "if", "for", "const", "return"}) m[t] = kKeyword;
+        return m;
+    }();
+    const auto it = words.find(w);
+    if (it != words.end()) return it->second;
+    return w.substr(0, 6) == "atomic" || vector_of_ints(w) ? kRefusedWord : kPlain;
+}
+
 // One logical line or the whole text into tokens; literals become one number
 // token "0" or, for strings, an identifier nothing accepts.
-void tokenize(const std::string &s, size_t i, size_t end, Toks &out)
+void tokenize(std::string_view s, size_t i, size_t end, Toks &out)
 {
-    static const char *three[] = {"<<=", ">>=", "..."};
-    static const char *two[] = {"++", "--", "+=", "-=", "*=", "/=", "%=", "&=", "|=", "^=", "==", "!=", "<=",
+    static const std::string_view three[] = {"<<=", ">>=", "..."};
+    static const std::string_view two[] = {"++", "--", "+=", "-=", "*=", "/=", "%=", "&=", "|=", "^=", "==", "!=", "<=",
                                 ">=", "&&", "||", "<<", ">>", "->", "##", "::"};
     while (i < end) {
         const char c = s[i];
@@ -36,55 +77,37 @@ void tokenize(const std::string &s, size_t i, size_t end, Toks &out)
         } else if (ident_start(c)) {
             size_t j = i + 1;
             while (j < end && ident_char(s[j])) ++j;
-            out.push_back({Kind::Ident, s.substr(i, j - i)});
+            out.push_back({Kind::Ident, s.substr(i, j - i), class_of(s.substr(i, j - i))});
             i = j;
         } else if (std::isdigit(static_cast<unsigned char>(c)) ||
                    (c == '.' && i + 1 < end && std::isdigit(static_cast<unsigned char>(s[i + 1])))) {
             size_t j = i + 1;
             while (j < end && (ident_char(s[j]) || s[j] == '.' ||
-                               ((s[j] == '+' || s[j] == '-') && std::string("eEpP").find(s[j - 1]) != std::string::npos)))
+                               ((s[j] == '+' || s[j] == '-') && std::string_view("eEpP").find(s[j - 1]) != std::string_view::npos)))
                 ++j;
             out.push_back({Kind::Number, s.substr(i, j - i)});
             i = j;
         } else if (c == '"' || c == '\'') {
             size_t j = i + 1;
             while (j < end && s[j] != c) j += (s[j] == '\\') ? 2 : 1;
-            out.push_back({Kind::Ident, "\"literal\""});
+            out.push_back({Kind::Ident, "\"literal\"", kRefusedWord});
             i = j + 1;
         } else {
-            std::string p(1, c);
-            for (const char *t : three)
-                if (s.compare(i, 3, t) == 0) p = t;
-            if (p.size() == 1)
-                for (const char *t : two)
-                    if (s.compare(i, 2, t) == 0) p = t;
+            size_t n = 1;
+            if (i + 1 < end && std::string_view("=+-&|<>:#.").find(s[i + 1]) != std::string_view::npos) {
+                for (const std::string_view t : three)
+                    if (s.substr(i, 3) == t) n = 3;
+                for (const std::string_view t : two)
+                    if (n == 1 && s.substr(i, 2) == t) n = 2;
+            }
+            const std::string_view p = s.substr(i, n);
             out.push_back({Kind::Punct, p});
             i += p.size();
         }
     }
 }
 
-const Names kIntTypes = {"int",   "unsigned", "signed", "long",   "short",    "char",      "size_t",   "ptrdiff_t",
-                         "uint",  "ulong",    "ushort", "uchar",  "intptr_t", "uintptr_t", "int8_t",   "int16_t",
-                         "int32_t", "int64_t", "uint8_t", "uint16_t", "uint32_t", "uint64_t", "wchar_t"};
-
-const Names kRefused = {"while",    "do",      "goto",  "switch",   "asm",       "__asm",    "__asm__",  "printf",
-                        "template", "union",   "enum",  "typedef",  "using",     "namespace", "class",   "struct",
-                        "auto",     "decltype", "typeof", "__typeof__", "operator", "new",    "delete",   "malloc",
-                        "free",     "try",     "throw", "volatile", "reinterpret_cast", "const_cast", "__builtin_assume",
-                        "sizeof",   "alignof", "extern", "\"literal\"", "__trap", "__syncthreads", "__syncwarp"};
-
-bool vector_of_ints(const std::string &w)  // int2, uchar4, longlong2, ...
-{
-    if (w.size() < 4 || !std::isdigit(static_cast<unsigned char>(w.back()))) return false;
-    size_t n = w.size();
-    while (n > 0 && std::isdigit(static_cast<unsigned char>(w[n - 1]))) --n;
-    std::string base = w.substr(0, n);
-    if (!base.empty() && base[0] == 'u') base.erase(0, 1);
-    return base == "int" || base == "long" || base == "longlong" || base == "short" || base == "char";
-}
-
-bool int_literal(const std::string &w)
+bool int_literal(std::string_view w)
 {
     const bool hex = w.size() > 2 && w[0] == '0' && (w[1] == 'x' || w[1] == 'X');
     for (const char c : w)
@@ -95,7 +118,7 @@ bool int_literal(const std::string &w)
 
 class Scan {
 public:
-    explicit Scan(const std::string &code)
+    explicit Scan(std::string_view code)
     {
         split(code);
         if (!hazard_.empty()) return;
@@ -106,7 +129,7 @@ public:
 
 private:
     struct Macro {
-        std::string name;
+        std::string_view name;
         Toks body;
     };
     struct Function {
@@ -120,7 +143,7 @@ private:
     Names index_ = {"_numeq_", "_numpar_", "_numnoi_", "_numsteps_", "_listsize_"};
     Names flags_;             // ints that hold a comparison
     Names tables_;            // arrays at file scope
-    std::map<std::string, Function> functions_;
+    std::map<std::string_view, Function> functions_;
     std::vector<char> allowed_;  // positions whose assignment a for header or a declaration makes
 
     bool refuse(const std::string &why)
@@ -128,14 +151,14 @@ private:
         if (hazard_.empty()) hazard_ = why;
         return false;
     }
-    bool is(size_t i, const char *s) const { return i < t_.size() && t_[i].text == s; }
+    bool is(size_t i, std::string_view s) const { return i < t_.size() && t_[i].text == s; }
     bool ident(size_t i) const { return i < t_.size() && t_[i].kind == Kind::Ident; }
     bool int_name(size_t i) const { return ident(i) && (index_.count(t_[i].text) || flags_.count(t_[i].text)); }
 
     // the matching closer of the opener at i, or npos
     size_t match(size_t i) const
     {
-        const std::string open = t_[i].text, close = open == "(" ? ")" : open == "[" ? "]" : "}";
+        const std::string_view open = t_[i].text, close = open == "(" ? ")" : open == "[" ? "]" : "}";
         int depth = 0;
         for (size_t k = i; k < t_.size(); ++k) {
             if (t_[k].text == open) ++depth;
@@ -167,7 +190,7 @@ private:
         bool found = false;
         int depth = 0;
         for (size_t k = a; k < b; ++k) {
-            const std::string &w = t_[k].text;
+            const std::string_view w = t_[k].text;
             if (w == "(" || w == "[") ++depth;
             else if (w == ")" || w == "]") --depth;
             else if (depth == 0) {
@@ -182,13 +205,13 @@ private:
     }
 
     // [a, b) at depth-0 commas
-    std::vector<std::pair<size_t, size_t>> pieces(size_t a, size_t b, const char *sep) const
+    std::vector<std::pair<size_t, size_t>> pieces(size_t a, size_t b, std::string_view sep) const
     {
         std::vector<std::pair<size_t, size_t>> out;
         int depth = 0;
         size_t from = a;
         for (size_t k = a; k < b; ++k) {
-            const std::string &w = t_[k].text;
+            const std::string_view w = t_[k].text;
             if (w == "(" || w == "[" || w == "{") ++depth;
             else if (w == ")" || w == "]" || w == "}") --depth;
             else if (depth == 0 && w == sep) {
@@ -201,7 +224,7 @@ private:
     }
 
     // directives out of the text; macro bodies behind it, each closed by ';'
-    void split(const std::string &s)
+    void split(std::string_view s)
     {
         const size_t n = s.size();
         size_t i = 0;
@@ -213,13 +236,12 @@ private:
             if (k < e && s[k] == '#') {
                 Toks d;
                 tokenize(s, k + 1, e, d);
-                const std::string what = d.empty() ? "" : d[0].text;
+                const std::string_view what = d.empty() ? std::string_view() : d[0].text;
                 if (what == "define") {
                     if (d.size() < 2 || d[1].kind != Kind::Ident) { refuse("#define"); return; }
-                    const std::string &name = d[1].text;
-                    if (kIntTypes.count(name) || name == "double" || name == "float" || name == "if" || name == "for" ||
-                        name == "const" || name == "return") {
-                        refuse("#define " + name);
+                    const std::string_view name = d[1].text;
+                    if (d[1].cls == kIntType || d[1].cls == kKeyword) {
+                        refuse("#define " + std::string(name));
                         return;
                     }
                     const size_t at = s.find(name, s.find("define", k) + 6) + name.size();
@@ -231,10 +253,10 @@ private:
                     }
                     Macro m{name, {}};
                     for (size_t q = from; q < d.size(); ++q) {
-                        if (d[q].text == "##" || d[q].text == "#") { refuse("#" + name); return; }
+                        if (d[q].text == "##" || d[q].text == "#") { refuse("#" + std::string(name)); return; }
                         m.body.push_back(d[q]);
                     }
-                    if (function) m.name.clear();  // never an index by itself
+                    if (function) m.name = {};  // never an index by itself
                     macros_.push_back(m);
                 } else if (what == "include" || what == "import" || what == "include_next") {
                     refuse("#include");
@@ -256,7 +278,7 @@ private:
     bool starts_statement(size_t i) const  // token i is the first of a statement
     {
         if (i == 0) return true;
-        const std::string &w = t_[i - 1].text;
+        const std::string_view w = t_[i - 1].text;
         return w == ";" || w == "{" || w == "}" || w == ")" || w == "else" || w == ":" || w == "static" || w == "inline";
     }
 
@@ -278,7 +300,7 @@ private:
                     for (const auto &p : pieces(i + 1, close, ",")) {
                         bool whole = false;
                         for (size_t k = p.first; k < p.second; ++k) {
-                            if (kIntTypes.count(t_[k].text)) whole = true;
+                            if ((t_[k].cls == kIntType)) whole = true;
                             if ((t_[k].text == "*" || t_[k].text == "&") && ident(k + 1)) f.pointers.insert(t_[k + 1].text);
                             if (t_[k].text == "[" && k > p.first && ident(k - 1)) f.pointers.insert(t_[k - 1].text);
                         }
@@ -309,11 +331,11 @@ private:
                 }
             }
             for (size_t i = 0; i < t_.size(); ++i) {
-                if (!kIntTypes.count(t_[i].text)) continue;
+                if (!(t_[i].cls == kIntType)) continue;
                 size_t first = i;
                 while (first > 0 && is(first - 1, "const")) --first;
                 size_t j = i;
-                while (j < t_.size() && (kIntTypes.count(t_[j].text) || is(j, "const"))) ++j;
+                while (j < t_.size() && ((t_[j].cls == kIntType) || is(j, "const"))) ++j;
                 if (!declare(first, j)) return;
                 i = j - 1;
             }
@@ -341,20 +363,20 @@ private:
         if (!in_for && !starts_statement(first)) return refuse("conversion to an integer type");
         for (size_t k = j;;) {
             if (!ident(k)) return refuse("integer declaration");
-            const std::string name = t_[k].text;
+            const std::string_view name = t_[k].text;
             size_t e = k + 1;
             if (is(e, "=")) {
                 int depth = 0;
                 size_t q = e + 1;
                 for (; q < t_.size(); ++q) {
-                    const std::string &w = t_[q].text;
+                    const std::string_view w = t_[q].text;
                     if (w == "(" || w == "[") ++depth;
                     else if (w == ")" || w == "]") --depth;
                     else if (depth == 0 && (w == "," || w == ";")) break;
                 }
                 if (!flags_.count(name) && index_expr(e + 1, q)) index_.insert(name);
                 else if (truth_expr(e + 1, q)) flags_.insert(name), index_.erase(name);
-                else if (!unresolved(e + 1, q)) return refuse("integer " + name + " from a value");
+                else if (!unresolved(e + 1, q)) return refuse("integer " + std::string(name) + " from a value");
                 allowed_[k] = 1;
                 e = q;
             } else if (!flags_.count(name)) {
@@ -374,7 +396,7 @@ private:
             if (t_[k].kind == Kind::Ident && !index_.count(t_[k].text)) return pending(t_[k].text);
         return false;
     }
-    bool pending(const std::string &name) const
+    bool pending(std::string_view name) const
     {
         for (const Macro &m : macros_)
             if (m.name == name) return true;
@@ -385,17 +407,17 @@ private:
     {
         int brace = 0;
         for (size_t i = 0; i < t_.size() && hazard_.empty(); ++i) {
-            const std::string &w = t_[i].text;
+            const std::string_view w = t_[i].text;
             if (w == "{") ++brace;
             if (w == "}") --brace;
             if (t_[i].kind == Kind::Ident) {
-                if (kRefused.count(w) || w.compare(0, 6, "atomic") == 0 || vector_of_ints(w)) { refuse(w); return; }
+                if (t_[i].cls == kRefusedWord) { refuse(w == "\"literal\"" ? "literal" : std::string(w)); return; }
                 if (w == "static" && brace > 0) { refuse("static"); return; }
                 if (w == "for") header(i);
                 // an int's name with another type elsewhere (the sets have no scopes)
-                if (i > 0 && ident(i - 1) && int_name(i) && !kIntTypes.count(t_[i - 1].text) && !is(i - 1, "const") &&
+                if (i > 0 && ident(i - 1) && int_name(i) && !(t_[i - 1].cls == kIntType) && !is(i - 1, "const") &&
                     !is(i - 1, "return") && !is(i - 1, "else"))
-                    refuse(w + " of two types");
+                    refuse(std::string(w) + " of two types");
                 if ((w == "double" || w == "float") && is(i + 1, "*") && brace > 0) { refuse("pointer"); return; }
                 const auto f = functions_.find(w);
                 if (f != functions_.end() && is(i + 1, "(") && i != f->second.begin) call(i, f->second);
@@ -408,16 +430,16 @@ private:
             if (w == "&" && int_name(i + 1) && i > 0 && t_[i - 1].kind == Kind::Punct && !is(i - 1, ")") && !is(i - 1, "]"))
                 refuse("address of an integer");
             // values: initialisers left open in collect
-            if (allowed_[i] && is(i + 1, "=") && index_.count(w) == 0 && flags_.count(w) == 0) refuse("integer " + w + " from a value");
+            if (allowed_[i] && is(i + 1, "=") && index_.count(w) == 0 && flags_.count(w) == 0) refuse("integer " + std::string(w) + " from a value");
         }
         for (size_t i = 0; i < t_.size() && hazard_.empty(); ++i) {
             const bool moved = assigned(i);
-            if (moved && int_name(i) && !allowed_[i]) refuse("assignment to integer " + t_[i].text);
+            if (moved && int_name(i) && !allowed_[i]) refuse("assignment to integer " + std::string(t_[i].text));
         }
         for (const auto &f : functions_)
             for (size_t i = f.second.begin; i < f.second.end && hazard_.empty(); ++i)
                 if (ident(i) && (f.second.pointers.count(t_[i].text) || tables_.count(t_[i].text)) && pointer_moved(i))
-                    refuse("pointer arithmetic on " + t_[i].text);
+                    refuse("pointer arithmetic on " + std::string(t_[i].text));
     }
 
     // an address other than an array's element is formed or assigned
@@ -445,7 +467,7 @@ private:
         const auto part = pieces(i + 2, close, ";");
         if (part.size() != 3) return refuse("for");
         size_t a = part[0].first;
-        while (a < part[0].second && (kIntTypes.count(t_[a].text) || is(a, "const"))) ++a;
+        while (a < part[0].second && ((t_[a].cls == kIntType) || is(a, "const"))) ++a;
         for (const auto &p : pieces(a, part[0].second, ",")) {
             if (!ident(p.first) || !index_.count(t_[p.first].text) || !is(p.first + 1, "=") || !index_expr(p.first + 2, p.second))
                 return refuse("for");
