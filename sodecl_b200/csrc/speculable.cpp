@@ -247,14 +247,18 @@ private:
                     const size_t at = s.find(name, s.find("define", k) + 6) + name.size();
                     const bool function = at < e && s[at] == '(';
                     size_t from = 2;
+                    Names arguments;
                     if (function) {
-                        while (from < d.size() && d[from].text != ")") ++from;
+                        for (; from < d.size() && d[from].text != ")"; ++from)
+                            if (d[from].kind == Kind::Ident) arguments.insert(d[from].text);
                         ++from;
                     }
                     Macro m{name, {}};
                     for (size_t q = from; q < d.size(); ++q) {
                         if (d[q].text == "##" || d[q].text == "#") { refuse("#" + std::string(name)); return; }
                         m.body.push_back(d[q]);
+                        // whatever it stands for, it is no int of the file's
+                        if (arguments.count(d[q].text)) m.body.back().text = "macro argument";
                     }
                     if (function) m.name = {};  // never an index by itself
                     macros_.push_back(m);
@@ -420,7 +424,10 @@ private:
                     refuse(std::string(w) + " of two types");
                 if ((w == "double" || w == "float") && is(i + 1, "*") && brace > 0) { refuse("pointer"); return; }
                 const auto f = functions_.find(w);
-                if (f != functions_.end() && is(i + 1, "(") && i != f->second.begin) call(i, f->second);
+                if (f != functions_.end() && i != f->second.begin) {
+                    if (is(i + 1, "(")) call(i, f->second);
+                    else refuse("function " + std::string(w) + " as a value");
+                }
             }
             if (w == "[") {
                 const size_t close = match(i);

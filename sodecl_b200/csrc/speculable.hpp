@@ -18,7 +18,7 @@ namespace sodecl_b200 {
 //    subscript, a bound or as an int argument): conversions, arrays of ints,
 //    functions that return them, assignments outside a for's header;
 //  - subscripts of anything but such ints; pointers other than parameters, and
-//    parameters that are moved; recursion;
+//    parameters that are moved; recursion, and functions as values;
 //  - and what the scan below does not follow: goto, switch, #include, type
 //    definitions, templates, inline assembly, printf.
 // The scan is of tokens, not of a syntax tree: it refuses some files that would

@@ -79,6 +79,10 @@ HELPERS = {
     "int result": "int at(double x) { return x > 0 ? 3 : 5; }\n" + HEAD + "\tyout[0] = p[at(exp(y[0]))];\n}\n",
     "two types": "double at(int k, double p[]) { return p[k]; }\ndouble sum(double k) { double s = 0; "
                  "for (int i = 0; i < k; i++) s += i; return s; }\n" + HEAD + "\tyout[0] = sum(exp(y[0])) + at(1, p);\n}\n",
+    "macro argument": "#define LOOP(n) for (int i = 0; i < n; i++) s += i;\ndouble at(int n, double p[]) { return p[n]; }\n" + HEAD +
+                      "\tdouble s = at(1, p);\n\tLOOP(exp(y[0]))\n\tyout[0] = s;\n}\n",
+    "function as a value": "double f(double x) { double (*g)(double) = f; return x > 1 ? g(x / 2) : x; }\n" + HEAD +
+                           "\tyout[0] = f(exp(y[0]));\n}\n",
     "recursion": "double f(double x) { return x > 1 ? f(x / 2) : x; }\n" + HEAD + "\tyout[0] = f(exp(y[0]));\n}\n",
     "typedef": "typedef int whole;\n" + HEAD + "\twhole k = exp(y[0]);\n\tyout[0] = p[k];\n}\n",
     "int array": "__constant int tab[3] = {0, 1, 2};\n" + HEAD + "\tyout[0] = exp(p[tab[1]]);\n}\n",
