@@ -629,10 +629,12 @@ int sodecl_cuda_device_describe(int device, char *buf, size_t n, int *major, int
         return SODECL_ERR_CUDA;
     }
     if (buf && n > 0) {
-        const int room = static_cast<int>(std::min<size_t>(n, 256));
-        buf[0] = '\0';
-        if (get_name(buf, room, device) != 0) return SODECL_ERR_CUDA;
-        buf[room - 1] = '\0';
+        // whole first: what the driver makes of a shorter buffer is its own affair
+        char name[256] = "";
+        if (get_name(name, sizeof name, device) != 0) return SODECL_ERR_CUDA;
+        name[sizeof name - 1] = '\0';
+        std::strncpy(buf, name, n - 1);
+        buf[n - 1] = '\0';
     }
     if (major) *major = cc[0];
     if (minor) *minor = cc[1];

@@ -50,3 +50,19 @@ def test_definitions_found(source, accepted, tmp_path):
     else:
         with pytest.raises(Exception, match="sode_system"):
             build()
+
+
+@pytest.mark.gpu
+def test_device_name_fits_any_buffer():
+    import ctypes as C
+
+    from sodecl_b200 import _native as N
+
+    whole = C.create_string_buffer(256)
+    major, minor = C.c_int(), C.c_int()
+    assert N.lib.sodecl_cuda_device_describe(0, whole, 256, C.byref(major), C.byref(minor)) == N.OK
+    assert len(whole.value) > 4 and major.value >= 10
+    for n in (1, 2, 5, len(whole.value), len(whole.value) + 1, 1000):
+        buf = C.create_string_buffer(b"x" * n, n)
+        assert N.lib.sodecl_cuda_device_describe(0, buf, n, None, None) == N.OK
+        assert buf.value == whole.value[:n - 1]
