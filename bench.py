@@ -379,10 +379,10 @@ def main():
                 "peak_source": "measured on this GPU: FMA-chain microbenchmark (sodecl_cuda_fma_peak, fastest of "
                                "7 launches), 2 flops/FMA",
                 "ops_per_orbit_step": RK4_OPS_PER_ORBIT_STEP,
-                "fp64_pipe_active": "52.4 % of peak (ncu sm__pipe_fp64_cycles_active, 2^18-orbit x 1000-step "
-                                    "launch of this kernel on this system file, dt 1e-3); counted source ops "
-                                    "understate the pipe work, exp and division expanding to many FP64 "
-                                    "instructions each"}
+                "fp64_pipe_active": "60.2 % of peak (ncu sm__pipe_fp64_cycles_active, 2^18-orbit x 500-step "
+                                    "launch of this kernel on the package's oculomotor file, dt 1e-3; 67.8 % at "
+                                    "dt 1e-6); counted source ops understate the pipe work, exp and division "
+                                    "expanding to many FP64 instructions each"}
 
     # ---------------- end to end through the C ABI with host buffers
     e2e = None
@@ -683,7 +683,7 @@ def tuning_steps(steps, scale=64):
 
 def sine_roofline(sines, seconds, peak, basis):
     """Roofline block of a Kuramoto line: sine evaluations per second against
-    the measured throughput of the math library's sin (sodecl_cuda_sin_peak,
+    the measured throughput of the programs' own sin (sodecl_cuda_sin_peak,
     fastest of 7 launches at full occupancy)."""
     achieved = sines / seconds
     return {"bound": "sin", "achieved": achieved, "peak": peak, "unit": "sines/s", "frac": achieved / peak,

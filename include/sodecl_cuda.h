@@ -68,8 +68,10 @@ extern "C" {
 /* how programs divide: SODECL_DIV_RECIPROCAL computes a/b as a*r plus two FMA
  * corrections with r = 1/b (hoistable out of the step loop for parameters and
  * constants), returns NaN at once for a NaN operand, and falls back to IEEE
- * division outside [2^-500, 2^500) (FP32: [2^-60, 2^60)): the same quotient as
- * SODECL_DIV_IEEE bit for bit (NaN payloads aside).  SODECL_DIV_DEFAULT (what
+ * division outside the range where that is exact ([2^-500, 2^500), FP32: [2^-60,
+ * 2^60); in speculative steps |a| in [2^-900, 2^900) by |b| in [2^-100, 2^100), FP32:
+ * [2^-102, 2^102) by [2^-24, 2^24)): the same quotient as SODECL_DIV_IEEE bit for
+ * bit (NaN payloads aside).  SODECL_DIV_DEFAULT (what
  * sodecl_cfg_init sets) is the reciprocal form in FP64 and IEEE division in
  * FP32 and for the adaptive solver.  On the oculomotor RK4 workload in FP64 the reciprocal form is 2 %
  * faster on converging orbits and 1.8x on diverged ones; in FP32 it gains on
@@ -108,8 +110,10 @@ typedef struct sodecl_cfg {
     int32_t record_f32;      /* device-API records stored as float (sodecl_cuda_launch only) */
     int32_t min_blocks_per_sm; /* launch-bounds occupancy hint for the compiler; 0 = default: none, except
                                   with one thread per orbit for the implicit and adaptive solvers,
-                                  which are held to 128 registers a thread, and for FP64 RK4 on up to
-                                  8 equations, held to 85 (1 lifts either) */
+                                  which are held to 128 registers a thread (the adaptive solver's
+                                  speculative program only where it does not spill), and for
+                                  FP64 RK4 on up to 8 equations, held to 85, or to 128 where its
+                                  steps are speculative (1 lifts either) */
     int32_t division;        /* quotients: SODECL_DIV_DEFAULT (the default: reciprocal in FP64, IEEE in
                                 FP32 and for SODECL_DORMAND_PRINCE), SODECL_DIV_RECIPROCAL or
                                 SODECL_DIV_IEEE;
@@ -448,16 +452,17 @@ void sodecl_batch_destroy(sodecl_batch *b);
 int sodecl_cuda_noise_stream(int device, const int64_t *gids, const double *counters, int64_t n, int32_t nnoi,
                              double dt_program, int64_t nsteps, double *normals, uint64_t *words, double *u01);
 
-/* Compares the reciprocal quotient of SODECL_DIV_RECIPROCAL with IEEE
- * division, bit for bit, on `pairs` pseudo-random operand pairs (every
+/* Compares the reciprocal quotient of SODECL_DIV_RECIPROCAL, and the quotients of
+ * speculative steps and of the banded solve in their ranges, with IEEE division,
+ * bit for bit, on `pairs` pseudo-random operand pairs (every
  * exponent, significands near 1 and 2, zeros, subnormals, Inf, NaN) drawn
  * from `seed`.  Writes the number of differing results and the first
  * differing pair. */
 int sodecl_cuda_division_check(int device, int64_t pairs, uint64_t seed, int64_t *mismatches, double *first_a,
                                double *first_b);
 
-/* The same for FP32 programs' reciprocal quotient (binary32, fast path for
- * |a|, |b| in [2^-60, 2^60)) against IEEE float division. */
+/* The same for FP32 programs' quotients (binary32; the reciprocal one's fast path
+ * for |a|, |b| in [2^-60, 2^60)) against IEEE float division. */
 int sodecl_cuda_division_check_f32(int device, int64_t pairs, uint64_t seed, int64_t *mismatches, float *first_a,
                                    float *first_b);
 
@@ -468,8 +473,8 @@ int sodecl_cuda_division_check_f32(int device, int64_t pairs, uint64_t seed, int
  * that launch's time. */
 int sodecl_cuda_fma_peak(int device, int32_t precision, double *fma_per_s, double *ms);
 
-/* Throughput microbenchmark of the math library's sin in FP64 (precision 0)
- * or FP32 (1): eight independent sums of sin(x_k - y) per thread on every SM,
+/* Throughput microbenchmark of the sine that solver programs take, in FP64
+ * (precision 0; without its range test) or FP32 (1; the math library's): eight independent sums of sin(x_k - y) per thread on every SM,
  * with arguments within a few units of zero, the coupling term of the
  * Kuramoto right-hand side.  Timed as sodecl_cuda_fma_peak; writes sines
  * per second and that launch's time.  It is the ceiling of a right-hand side

@@ -268,8 +268,9 @@ def fma_peak(precision="fp64", device=0):
 
 
 def sin_peak(precision="fp64", device=0):
-    """Measured sine evaluations per second of the math library's sin (FP64 or
-    FP32) at full occupancy, arguments within a few units of zero."""
+    """Measured sine evaluations per second of the programs' sine (FP64: the
+    straight-line one; FP32: the math library's) at full occupancy, arguments
+    within a few units of zero."""
     rate, ms = C.c_double(), C.c_double()
     prec = N.FP32 if precision == "fp32" else N.FP64
     N.check(N.lib.sodecl_cuda_sin_peak(device, prec, C.byref(rate), C.byref(ms)))

@@ -4,8 +4,8 @@
 //    tests against the CPU generator;
 //  * an FMA issue-rate microbenchmark, the denominator of the FP64/FP32
 //    "fraction of issue peak" figures;
-//  * a check of the reciprocal quotient (device/fastdiv.cuh) against IEEE
-//    division on random and special operands.
+//  * a check of the reciprocal and the straight-line quotients
+//    (device/fastdiv.cuh) against IEEE division on random and special operands.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -91,8 +91,16 @@ __global__ void division_check_kernel(unsigned long long seed, long long per_thr
     unsigned long long bad = 0;
     for (long long i = 0; i < per_thread; ++i) {
         const double a = division_operand(state), b = division_operand(state);
-        const double want = a / b, got = sodecl_div_rcp(a, b);
-        const bool same = (__double_as_longlong(want) == __double_as_longlong(got)) || (want != want && got != got);
+        const double want = a / b;
+        const auto is_it = [want](double got) {
+            return __double_as_longlong(want) == __double_as_longlong(got) || (want != want && got != got);
+        };
+        // the guarded quotient, and the straight-line ones where they say they hold
+        bool same = is_it(sodecl_div_rcp(a, b)), outside = false;
+        const double chain = sodecl_div_chain(a, b, outside);
+        same = same && (outside || is_it(chain));
+        outside = sodecl_straight_divisor_outside(b) || sodecl_straight_dividend_outside(a);
+        same = same && (outside || is_it(sodecl_div_straight(a, b, 1.0 / b)));
         if (!same) {
             if (atomicAdd(mismatches, 1ULL) == 0) {
                 first[0] = a;
@@ -136,8 +144,12 @@ __global__ void division_check_f32_kernel(unsigned long long seed, long long per
     unsigned long long state = seed ^ (0xD1B54A32D192ED03ULL * (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x + 1));
     for (long long i = 0; i < per_thread; ++i) {
         const float a = division_operand_f32(state), b = division_operand_f32(state);
-        const float want = a / b, got = sodecl_div_rcp(a, b);
-        const bool same = (__float_as_int(want) == __float_as_int(got)) || (want != want && got != got);
+        const float want = a / b;
+        const auto is_it = [want](float got) {
+            return __float_as_int(want) == __float_as_int(got) || (want != want && got != got);
+        };
+        const bool outside = sodecl_straight_divisor_outside(b) || sodecl_straight_dividend_outside(a);
+        const bool same = is_it(sodecl_div_rcp(a, b)) && (outside || is_it(sodecl_div_straight(a, b, 1.0f / b)));
         if (!same && atomicAdd(mismatches, 1ULL) == 0) {
             first[0] = a;
             first[1] = b;
@@ -164,7 +176,11 @@ __global__ void __launch_bounds__(256) fma_chains_kernel(T *sink, int iters, T a
 
 // Sines at full occupancy: eight independent sums of sin(x_k - y) per thread,
 // the coupling term of a Kuramoto row, with arguments within a few units of
-// zero (where phases that have drifted apart by a few radians put them).
+// zero (where phases that have drifted apart by a few radians put them).  The
+// sine is the solver programs': in FP64 the straight-line one, in FP32 the
+// library's.
+__device__ __forceinline__ double program_sine(double x) { return sodecl_sin_core(x); }
+__device__ __forceinline__ float program_sine(float x) { return sin(x); }
 template <class T>
 __global__ void __launch_bounds__(256) sin_sums_kernel(T *sink, int iters, T step)
 {
@@ -178,7 +194,7 @@ __global__ void __launch_bounds__(256) sin_sums_kernel(T *sink, int iters, T ste
     T y = (T)0;
     for (int i = 0; i < iters; ++i) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] += sin(x[k] - y);
+        for (int k = 0; k < 8; ++k) acc[k] += program_sine(x[k] - y);
         y += step;
     }
     const T s = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
