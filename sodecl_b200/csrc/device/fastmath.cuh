@@ -115,31 +115,45 @@ __device__ __forceinline__ void sodecl_lower()
     SODECL_MATH_AS_DOUBLE(name, long long)                                                     \
     SODECL_MATH_AS_DOUBLE(name, unsigned long long)                                            \
     SODECL_MATH_NUM(name)
-// sincos in both its forms (OpenCL's and CUDA's): the values of sin and cos
-#define SODECL_MATH_SINCOS(name, sine, cosine, type)                                           \
-    __device__ __forceinline__ type name(type x, type *c)                                      \
+// sincos in both its forms (OpenCL's and CUDA's): the values of sin and cos, from
+// one reduction and with one test
+template <bool Raise, bool Library> __device__ __forceinline__ double sodecl_sincos_of(double x, double *c)
+{
+    bool outside;
+    double cosine;
+    const double sine = sodecl_sincos_bounded(x, cosine, outside);
+    if (Raise) sodecl_raise(outside);
+    const bool library = Library && outside;
+    *c = library ? ::cos(x) : cosine;
+    return library ? ::sin(x) : sine;
+}
+template <bool Raise, bool Library> __device__ __forceinline__ float sodecl_sincos_of(float x, float *c)
+{
+    *c = ::cos(x);
+    return ::sin(x);
+}
+#if SODECL_FAST_DIV
+template <bool Raise, bool Library> __device__ __forceinline__ sodecl_num sodecl_sincos_of(sodecl_num x, sodecl_num *c)
+{
+    return sodecl_num(sodecl_sincos_of<Raise, Library>(x.v, &c->v));
+}
+#endif
+#define SODECL_MATH_SINCOS(name, raise, library)                                               \
+    template <class X, class R> __device__ __forceinline__ R name(X x, R *c)                   \
     {                                                                                          \
-        *c = cosine(x);                                                                        \
-        return sine(x);                                                                        \
+        return sodecl_sincos_of<raise, library>((R)x, c);                                      \
     }                                                                                          \
-    __device__ __forceinline__ void name(type x, type *s, type *c)                             \
+    template <class X, class R> __device__ __forceinline__ void name(X x, R *s, R *c)          \
     {                                                                                          \
-        *s = sine(x);                                                                          \
-        *c = cosine(x);                                                                        \
+        *s = sodecl_sincos_of<raise, library>((R)x, c);                                        \
     }
 
 SODECL_MATH_FN(sin, ::sin)
 SODECL_MATH_FN(cos, ::cos)
 SODECL_MATH_FN(exp, ::exp)
-#define SODECL_MATH_SINCOS_OF(type)                                                            \
-    SODECL_MATH_SINCOS(sodecl_spec_sincos, sodecl_spec_sin, sodecl_spec_cos, type)             \
-    SODECL_MATH_SINCOS(sodecl_plain_sincos, sodecl_plain_sin, sodecl_plain_cos, type)          \
-    SODECL_MATH_SINCOS(sodecl_full_sincos, sodecl_full_sin, sodecl_full_cos, type)
-SODECL_MATH_SINCOS_OF(double)
-SODECL_MATH_SINCOS_OF(float)
-#if SODECL_FAST_DIV
-SODECL_MATH_SINCOS_OF(sodecl_num)
-#endif
+SODECL_MATH_SINCOS(sodecl_spec_sincos, true, false)
+SODECL_MATH_SINCOS(sodecl_plain_sincos, true, true)
+SODECL_MATH_SINCOS(sodecl_full_sincos, false, true)
 
 #if SODECL_FAST_DIV
 // The IEEE quotient's bits.  The divisor's test is a branch of its own: it keeps

@@ -146,6 +146,15 @@ __device__ __forceinline__ double sodecl_cos_bounded(double x, bool &outside)
     return __hiloint2double(outside ? 0 : __double2hiint(v), __double2loint(v));
 }
 
+__device__ __forceinline__ double sodecl_sincos_bounded(double x, double &cosine, bool &outside)
+{
+    const sodecl_quarter q = sodecl_quarter_of(x);
+    const double s = sodecl_quarter_sin(q, q.n), c = sodecl_quarter_sin(q, q.n + 1);
+    outside = sodecl_trig_outside(x);
+    cosine = __hiloint2double(outside ? 0 : __double2hiint(c), __double2loint(c));
+    return __hiloint2double(outside ? 0 : __double2hiint(s), __double2loint(s));
+}
+
 // exp is 0 from -748 down and infinity from 748 up, and outside only between
 // them and 708.  The high word as a float is ordered like the number: 4.19140625f
 // is that of 708, 4.23046875f that of 748; those of the largest numbers, Inf and

@@ -96,6 +96,8 @@ SAFE = {
              "\tconst int n = LAST;\n\tfor (int i = 0; i <= n; i += 1) yout[i] = exp(-y[i]) / 3;\n}\n",
     "helper": "double row(int i, const double *y) { double c; double s = sincos(y[i], &c); return s * c; }\n" + HEAD +
               "\tfor (int i = 0; i < _numeq_; i++) yout[i] = row(i, y);\n}\n",
+    "sincos": HEAD + "\tdouble a, b, c;\n\tfloat d;\n\ta = sincos(y[0], &b);\n\tsincos(y[1], &a, &c);\n\tsincos(1, &b);\n"
+              "\tsincos(0.5f * _numeq_, &c);\n\tsincos(0.5f, &d);\n\tyout[0] = a + b * c + d;\n}\n",
     "prototype": "double f(double x);\ndouble f(double x) { return exp(x); }\n" + HEAD + "\tyout[0] = f(y[0]);\n}\n",
     "comments": "// while (1)\n" + HEAD + "\t/* int k = exp(1); goto */\n" + PLAIN + "}\n",
     "table": "__constant double tab[3] = {1.0, 2.0, 3.0};\n" + HEAD + "\tyout[0] = exp(-tab[2] * y[0]);\n}\n",
