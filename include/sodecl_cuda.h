@@ -111,7 +111,7 @@ typedef struct sodecl_cfg {
     int32_t min_blocks_per_sm; /* launch-bounds occupancy hint for the compiler; 0 = default: none, except
                                   with one thread per orbit for the implicit and adaptive solvers,
                                   which are held to 128 registers a thread (the adaptive solver's
-                                  speculative program only where it does not spill), and for
+                                  speculative program is not), and for
                                   FP64 RK4 on up to 8 equations, held to 85, or to 128 where its
                                   steps are speculative (1 lifts either) */
     int32_t division;        /* quotients: SODECL_DIV_DEFAULT (the default: reciprocal in FP64, IEEE in

@@ -757,44 +757,6 @@ std::shared_ptr<const Program> compile_one(const ProgramSpec &spec, const std::s
                         spec.fast_math == FastMath::Speculative);
 }
 
-// The sum over the program's functions of a figure of the compiler's report
-// (" bytes spill stores": registers stored to local memory).
-int reported_bytes(const Program &prog, const char *marker)
-{
-    int sum = 0;
-    for (size_t at = prog.log.find(marker); at != std::string::npos; at = prog.log.find(marker, at + 1)) {
-        size_t digits = at;
-        while (digits > 0 && prog.log[digits - 1] >= '0' && prog.log[digits - 1] <= '9') --digits;
-        sum += std::atoi(prog.log.c_str() + digits);
-    }
-    return sum;
-}
-
-// `capped`, or the program without the register cap where only that keeps
-// everything in registers.  The attempts of the adaptive solver's speculative
-// program (few orbits: kLatencyOrbits) are one long chain for each lane, so what
-// spills on it counts and occupancy hardly: oculomotor 12.0 ms without the cap (222
-// registers) against 15.5 with it (542 bytes spilt) at 4097 orbits over 0.02 time
-// units, 38.8 against 50.6 at 2^14 over 0.2, 74.3 against 83.8 at 2^17.  Up to 128
-// bytes, some 16 of the cap's 128 registers, stay in the first-level cache next to
-// the chain's quotients and occupancy is worth as much (Kuramoto of 5 phases, 16
-// bytes: 1.30 with the cap, 1.24 without at 2^14 orbits, 3.35 and 3.94 at 2^17);
-// and where the uncapped program keeps more than the math library's slow path in
-// local memory all the same (40 bytes), the state is not in registers either.
-std::shared_ptr<const Program> compile_uncapped(const ProgramSpec &spec, const std::string &system_src,
-                                                const SystemTraits &traits, std::shared_ptr<const Program> capped)
-{
-    if (!spec.default_cap || spec.solver != 5 || spec.fast_math != FastMath::Speculative ||
-        reported_bytes(*capped, " bytes spill stores") <= 128)
-        return capped;
-    ProgramSpec free = spec;
-    free.min_blocks = 1;
-    auto uncapped = compile_one(free, system_src, traits);
-    const bool resident = reported_bytes(*uncapped, " bytes spill stores") == 0 &&
-                          reported_bytes(*uncapped, " bytes stack frame") <= 64;
-    return resident ? uncapped : capped;
-}
-
 }  // namespace
 
 int batch_warp_words(const std::vector<BatchClass> &classes)
@@ -986,9 +948,14 @@ std::shared_ptr<const Program> build(const ProgramSpec &spec, const std::string 
             // 1000 steps: 31.6 ms so, 28.7 at 128 registers)
             if (t.default_cap && t.solver == 2 && t.fast_math == FastMath::Speculative)
                 t.min_blocks = std::max(1, 65536 / (t.block_max * 128));
+            // the adaptive solver, where it speculates: launches that wait for their
+            // longest chains, on which a spilt register is a load (oculomotor, 128
+            // registers and 542 bytes spilt against 224: 15.5 / 12.0 ms at 4097 orbits
+            // over 0.02 time units, 50.6 / 38.8 at 2^14 over 0.2, 83.8 / 74.3 at 2^17)
+            if (t.default_cap && t.solver == 5 && t.fast_math == FastMath::Speculative) t.min_blocks = 1;
             if (!fast_div && !math) return compile_one(t, system_src, traits);
             try {
-                return compile_uncapped(t, system_src, traits, compile_one(t, system_src, traits));
+                return compile_one(t, system_src, traits);
             } catch (const std::exception &e) {
                 if (math) why = first_error(e.what());
             }

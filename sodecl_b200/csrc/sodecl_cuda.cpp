@@ -532,8 +532,8 @@ ProgramSpec make_spec(const sodecl_cfg &c)
     // implicit solvers, one thread per orbit: by default at most 128 registers
     // a thread (four blocks of 128 threads on an SM); above that the Newton
     // pass's hoisted terms took more registers than the occupancy they cost
-    // The adaptive solver's kernel likewise, unless the cap makes its
-    // speculative attempts spill registers (program.cpp, build)
+    // The adaptive solver's kernel likewise, unless it speculates (program.cpp,
+    // build)
     if (spec.min_blocks == 0 && lanes_of(c) == 1 &&
         (c.solver == SODECL_IMPLICIT_EULER || c.solver == SODECL_IMPLICIT_MIDPOINT ||
          c.solver == SODECL_DORMAND_PRINCE)) {
