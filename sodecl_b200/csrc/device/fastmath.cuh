@@ -21,7 +21,8 @@
 // not depend on where a run, a launch or a record interval began.  After a plain
 // step the next one is tried with the plain copy first; it counts if it raises
 // the flag too, else the speculative copy decides again.  So an orbit that stays
-// outside pays for the plain copy alone.
+// outside pays for the plain copy alone (in FP32 with IEEE division for both: float's
+// own quotients raise no flag).
 // Programs without speculative steps (the one-thread implicit kernel) call
 // sodecl_full_sin and so on, the plain copy's values without the flag.
 #ifndef SODECL_FASTMATH_CUH

@@ -30,9 +30,9 @@
 //   SODECL_HAS_ROW_BAND  the system file defines sode_system_row_band
 //   SODECL_PAIR_STORES   one-thread kernel: records written two orbits per
 //                        vector store (sodecl_store_pairs)
-//   SODECL_SPECULATE     explicit and stochastic solvers, implicit solvers with
-//                        lanes per orbit: steps run on the speculative copy
-//                        of the system file (fastmath.cuh), which with this
+//   SODECL_SPECULATE     explicit, stochastic and adaptive solvers, implicit
+//                        solvers with lanes per orbit: steps (attempts) run on
+//                        the speculative copy of the system file (fastmath.cuh), which with this
 //                        file's step functions lies in namespace sodecl_spec
 //                        (SODECL_SPEC_COPY, assembled first)
 

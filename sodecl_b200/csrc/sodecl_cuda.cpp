@@ -541,7 +541,8 @@ ProgramSpec make_spec(const sodecl_cfg &c)
         spec.default_cap = c.solver == SODECL_DORMAND_PRINCE;
     }
     // FP64 RK4 on small systems, one thread per orbit: by default at most 85
-    // registers a thread (three blocks of 256).  Measured on the oculomotor
+    // registers a thread (three blocks of 256), 128 where its steps are
+    // speculative (program.cpp, build).  Measured on the oculomotor
     // model at 2^20 orbits x 10^4 steps: 397 ms against 426 ms with no cap
     // and 411 ms at 64 registers (the reference's system file; the package's
     // 362 / 381 / 371 ms).
